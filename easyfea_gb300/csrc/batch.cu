@@ -536,8 +536,7 @@ __device__ void solve_instance(Ctx& c, const gfea_batch_instance& I, double delt
       else
         restart_rz<D, T>(I, w, gtid, nthr, vz);
       csum<2>(c, vz, oz);
-      beta = oz[0] / rz;
-      if (!(beta <= 1.0)) beta = 0;  // a replaced residual above the iterated one restarts
+      beta = next_beta(2, oz[0], rz, beta);
       rz = oz[0];
       trigger = fmax(delta2 * rr_true, 0.25 * tol2);
     }

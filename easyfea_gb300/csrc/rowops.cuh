@@ -248,4 +248,19 @@ __device__ __forceinline__ A node_rows_s(const T* vrow, const int32_t* nrow, int
   return group_sum_rows<D, G, A>(acc, lane);
 }
 
+// beta of the next search direction p = z + beta p_old from this residual's
+// r.z and the previous one's.  mode 0: PCG iteration; mode 1: start; mode 2:
+// the iterated residual was replaced (reliable update) after its iteration
+// had set beta = rz / rz_before, so r.z takes rz's place in that ratio.
+// (Dividing by the iterated residual's own rz gives a beta near 1 whatever
+// the iteration's was, which loses conjugacy: the 208-unknown cantilever took
+// 98-148 iterations instead of 46.)  A replaced residual far above the
+// iterated one (drift) restarts the direction.
+__device__ __forceinline__ double next_beta(int mode, double rz_new, double rz, double beta) {
+  if (mode == 1) return 0.0;
+  const double ratio = rz_new / rz;
+  if (mode == 0) return ratio;
+  return ratio <= 4.0 ? beta * ratio : 0.0;
+}
+
 }  // namespace gfea

@@ -315,7 +315,7 @@ __global__ void bjacobi_kernel(SysT<T> S, T* __restrict__ dinv, int32_t* flag) {
 // z = D^-1 r, partial r.z and r.r; the last block derives beta and the
 // convergence state.  mode 0: PCG iteration (x += alpha p, r -= alpha Ap
 // first); mode 1: start (beta = 0); mode 2: residual replaced by a reliable
-// update (beta = r.z / previous r.z, the search direction is kept).
+// update (the search direction is kept, see next_beta).
 template <int D, typename T>
 __global__ void __launch_bounds__(kThreads) update_kernel(int64_t Nn, const uint8_t* __restrict__ known,
                                                           const T* __restrict__ dinv, T* __restrict__ x,
@@ -353,9 +353,7 @@ __global__ void __launch_bounds__(kThreads) update_kernel(int64_t Nn, const uint
   double out[2];
   if (reduce_last_acc<2, T>(v, partials, &sc->ticket2, out) && threadIdx.x == 0) {
     const double rz_new = out[0], rr = out[1];
-    sc->beta = mode == 1 ? 0.0 : rz_new / sc->rz;
-    // a replaced residual larger than the iterated one (drift) restarts the direction
-    if (mode == 2 && !(sc->beta <= 1.0)) sc->beta = 0.0;
+    sc->beta = next_beta(mode, rz_new, sc->rz, sc->beta);
     sc->rz = rz_new;
     sc->rr = rr;
     if (mode != 0) return;  // the host sets the next stopping threshold
@@ -835,8 +833,7 @@ __global__ void __launch_bounds__(kThreads) finish_z_kernel(int64_t Nn, const ui
   double out[2];
   if (reduce_last_acc<2, T>(v, partials, &sc->ticket2, out) && threadIdx.x == 0) {
     const double rz_new = out[0], rr = out[1];
-    sc->beta = mode == 1 ? 0.0 : rz_new / sc->rz;
-    if (mode == 2 && !(sc->beta <= 1.0)) sc->beta = 0.0;
+    sc->beta = next_beta(mode, rz_new, sc->rz, sc->beta);
     sc->rz = rz_new;
     sc->rr = rr;
     if (mode != 0) return;
