@@ -263,4 +263,24 @@ __device__ __forceinline__ double next_beta(int mode, double rz_new, double rz, 
   return ratio <= 4.0 ? beta * ratio : 0.0;
 }
 
+// Row j of the node from the partial rows of its D component lanes: in step
+// s the lane of component j' offers its partial of row (j' - s) mod D, and
+// the lane of component j takes the offer of lane j + s (mod D).
+template <int D, typename T>
+__device__ __forceinline__ T node_rows_exchange(const T (&acc)[D], int j, int lane) {
+  T row = acc[0];
+#pragma unroll
+  for (int i = 1; i < D; ++i) row = (j == i) ? acc[i] : row;
+#pragma unroll
+  for (int st = 1; st < D; ++st) {
+    const int oi = j >= st ? j - st : j - st + D;  // (j - st) mod D
+    const int sj = j + st < D ? j + st : j + st - D;  // (j + st) mod D
+    T offer = acc[0];
+#pragma unroll
+    for (int i = 1; i < D; ++i) offer = (oi == i) ? acc[i] : offer;
+    row += __shfl_sync(0xffffffffu, offer, lane - j + sj);
+  }
+  return row;
+}
+
 }  // namespace gfea

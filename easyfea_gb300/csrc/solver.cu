@@ -35,6 +35,8 @@
 
 #include "coarse.cuh"
 #include "common.cuh"
+#include "pcg_types.cuh"
+#include "resident.cuh"
 #include "rowops.cuh"
 #include "stage.cuh"
 #include "tune.cuh"
@@ -383,43 +385,6 @@ __global__ void __launch_bounds__(kThreads) update_kernel(int64_t Nn, const uint
 
 constexpr int kCoarseMax = 1536;  // largest coarse dimension nr * n_agg
 
-// Aggregation kept at the start of the coarse workspace, so that a later
-// solve on the same mesh can reuse it.
-struct CoarseHdr {
-  int32_t n_agg, nc, nr, valid;
-  int64_t Nn;
-};
-
-// The restriction's FP64 atomics go to kRcCopies copies of the coarse vector
-// (block b adds into copy b % kRcCopies): one copy held them all on a few L2
-// slices, where they serialised.  Below kRcCopyMinNodes nodes the atomics
-// are few and an iteration is launch-latency bound: one copy (rc itself,
-// cleared by finish_z) and no summing launch.
-constexpr int kRcCopies = 16;
-constexpr int64_t kRcCopyMinNodes = 100000;
-
-struct CoarseDev {
-  int nr = 0, n_agg = 0, nc = 0;
-  int ncopies = 1;         // 1: restriction into rc; kRcCopies: into rcp, summed by rc_sum_kernel
-  CoarseHdr* hdr = nullptr;
-  int32_t* agg = nullptr;  // node -> aggregate
-  float4* off = nullptr;   // node offset from its cell centre / largest cell size
-  double* Ac = nullptr;    // nc x nc, inverted in place
-  // working storage of the inversion: float-float pairs (hi, lo)
-  float* Ahi = nullptr;    // nc x nc
-  float* Alo = nullptr;
-  float* rowph = nullptr;  // kGJB x nc: row panel of the pivot block
-  float* rowpl = nullptr;
-  float* colph = nullptr;  // nc x kGJB: column panel of the pivot block
-  float* colpl = nullptr;
-  float* pinvh = nullptr;  // kGJB x kGJB: inverse of the pivot block
-  float* pinvl = nullptr;
-  double* rc = nullptr;    // nc: restriction R^T r (summed from the copies)
-  double* rcp = nullptr;   // kRcCopies x nc: restriction accumulators, one per group of blocks
-  double* ec = nullptr;    // nc: coarse correction
-  float* ecf = nullptr;    // nc: its FP32 copy (read by the FP32 prolongation)
-};
-
 __global__ void bbox_kernel(const double* __restrict__ coord, int64_t Nn, double* partials) {
   double lo[3] = {INFINITY, INFINITY, INFINITY}, hi[3] = {-INFINITY, -INFINITY, -INFINITY};
   for (int64_t a = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; a < Nn; a += (int64_t)gridDim.x * blockDim.x)
@@ -687,26 +652,6 @@ __device__ __forceinline__ void gj_update_body(const CoarseDev& C, int k0, int b
 
 __global__ void __launch_bounds__(128) gj_update_kernel(CoarseDev C, int k0, int b) {
   gj_update_body(C, k0, b, blockIdx.x, blockIdx.y, gridDim.y);
-}
-
-template <int nr, typename T>
-__device__ __forceinline__ void restrict_add(double* rc, int g, T (&v)[nr]) {
-  const int lane = threadIdx.x & 31;
-  const int gp = __shfl_up_sync(0xffffffffu, g, 1);
-  const unsigned heads = __ballot_sync(0xffffffffu, lane == 0 || g != gp);
-  const int start = 31 - __clz(heads & (0xffffffffu >> (31 - lane)));  // first lane of this lane's run
-  const int gn = __shfl_down_sync(0xffffffffu, g, 1);
-  const bool tail = lane == 31 || gn != g;
-#pragma unroll
-  for (int m = 0; m < nr; ++m) {
-    T s = v[m];
-#pragma unroll
-    for (int d = 1; d < 32; d <<= 1) {
-      const T t = __shfl_up_sync(0xffffffffu, s, d);
-      if (lane - d >= start) s += t;
-    }
-    if (tail && g >= 0 && s != 0) atomicAdd(&rc[g * nr + m], (double)s);
-  }
 }
 
 // x, r update (mode 0) and restriction rc += R_a^T r_a.  The node loop runs
@@ -982,26 +927,6 @@ __global__ void __launch_bounds__(kThreads) pack_tiles_kernel(SysT<T> S, StageGe
         if (e + 32 * u < n) V[e + 32 * u] = v[u];
     }
   }
-}
-
-// Row j of the node from the partial rows of its D component lanes: in step
-// s the lane of component j' offers its partial of row (j' - s) mod D, and
-// the lane of component j takes the offer of lane j + s (mod D).
-template <int D, typename T>
-__device__ __forceinline__ T node_rows_exchange(const T (&acc)[D], int j, int lane) {
-  T row = acc[0];
-#pragma unroll
-  for (int i = 1; i < D; ++i) row = (j == i) ? acc[i] : row;
-#pragma unroll
-  for (int st = 1; st < D; ++st) {
-    const int oi = j >= st ? j - st : j - st + D;  // (j - st) mod D
-    const int sj = j + st < D ? j + st : j + st - D;  // (j + st) mod D
-    T offer = acc[0];
-#pragma unroll
-    for (int i = 1; i < D; ++i) offer = (oi == i) ? acc[i] : offer;
-    row += __shfl_sync(0xffffffffu, offer, lane - j + sj);
-  }
-  return row;
 }
 
 // Partial rows (all D rows, component j) of node a over its nb neighbours:
@@ -1317,6 +1242,7 @@ struct PcgWork {
   bool is_f32 = false;  // T-typed buffers hold floats
   CoarseDev C;
   unsigned char* packed = nullptr;  // tiles of the staged SpMV (nullptr: apply_kernel)
+  unsigned char* box = nullptr;     // packets of the resident solve (nullptr: the multi-kernel iteration)
   StageGeom geom{};
   // CUDA graphs of kGraphIters PCG iterations, one per direction-buffer order
   cudaGraphExec_t gexec[2] = {nullptr, nullptr};
@@ -1334,8 +1260,6 @@ struct PcgWork {
   }
 };
 
-int coarse_nr(int D) { return D == 1 ? 1 : (D == 2 ? 3 : 6); }
-
 // Number of aggregates of the coarse level (0: block-Jacobi only).
 // Automatic: k Nn^0.43 (k = 0.6 for 3D elasticity, 1.5 otherwise), which
 // balances the coarse inverse (~ nc^3) against the iterations it saves
@@ -1351,7 +1275,7 @@ int coarse_target(const gfea_system* s, const gfea_pcg_opts* o) {
 }
 
 template <typename T>
-size_t pcg_layout(int64_t Nn, int D, int n_agg_max, PcgWork* w, char* base, size_t packed = 0) {
+size_t pcg_layout(int64_t Nn, int D, int n_agg_max, PcgWork* w, char* base, size_t packed = 0, size_t box = 0) {
   size_t off = 0;
   const int64_t N = Nn * D;
   auto take = [&](size_t bytes) {
@@ -1395,6 +1319,7 @@ size_t pcg_layout(int64_t Nn, int D, int n_agg_max, PcgWork* w, char* base, size
     w->C.ecf = reinterpret_cast<float*>(take(sizeof(float) * nc));
   }
   w->packed = packed ? reinterpret_cast<unsigned char*>(take(packed)) : nullptr;
+  w->box = box ? reinterpret_cast<unsigned char*>(take(box)) : nullptr;
   return off;
 }
 
@@ -2052,6 +1977,30 @@ int fetch(Scal* h, PcgWork& w, cudaStream_t st) {
   return GFEA_OK;
 }
 
+// Whether this solve runs as one resident launch (resident.cu): an operator
+// that is not staged (its tiles would fit in half of the L2), host checks left
+// to the library, and nothing that needs the iteration's launches one by one
+// (kernel timing, a first solve that tunes the SpMV, the direct-launch entry).
+template <typename T>
+bool use_resident(const gfea_system* s, const gfea_pcg_opts* o, const PcgWork& w, bool direct_only, ResidentGeom* g) {
+  if (direct_only || !w.box || o->check_every > 0 || prof().on.load()) return false;
+  static const bool off = [] {
+    const char* v = getenv("GFEA_RESIDENT");  // "0": the multi-kernel iteration
+    return v && v[0] == '0';
+  }();
+  if (off) return false;
+  int32_t tuned = 0;
+  if (o->lanes == 0 && tune_cache().mode.load() == 2 && !tune_get(spmv_key(s, sizeof(T) == 4 ? GFEA_F32 : GFEA_F64), &tuned))
+    return false;
+  // Solves in flight share the SMs: a cooperative grid starts when all its
+  // CTAs fit, so full-size grids would run one after the other, each bound by
+  // latency (24 served requests: 55 ms with full-size grids, 39 ms with a
+  // share each, 48 ms with the multi-kernel iteration).
+  const int active = std::min(std::max(active_solves().load(), 1), 4);
+  return resident_geom<T>(s->dof_n, s->n_nodes, s->n_pairs, w.coarse ? w.C.nc : 0, w.coarse ? w.C.n_agg : 0,
+                          kSMs / active, g);
+}
+
 // PCG in T precision with reliable updates (FP64 residual replacement):
 //   the iteration runs on T values and vectors with FP64 dots and scalar
 //   recurrences, accumulating its correction in dx; whenever the iterated
@@ -2073,7 +2022,9 @@ int refine_solve(const gfea_system* s, const double* b, double* x, const gfea_pc
   size_t pk = packed_bytes<T>(s);
   if (const char* e = getenv("GFEA_APPLY_STAGED")) if (e[0] == '0') pk = 0;  // the unstaged kernel (A/B runs)
   if (pk && pcg_layout<T>(s->n_nodes, s->dof_n, target, nullptr, nullptr, pk) > work_bytes) pk = 0;
-  if (pcg_layout<T>(s->n_nodes, s->dof_n, target, &w, static_cast<char*>(work), pk) > work_bytes)
+  size_t box = pk || direct_only ? 0 : kResidentBox;
+  if (box && pcg_layout<T>(s->n_nodes, s->dof_n, target, nullptr, nullptr, pk, box) > work_bytes) box = 0;
+  if (pcg_layout<T>(s->n_nodes, s->dof_n, target, &w, static_cast<char*>(work), pk, box) > work_bytes)
     return GFEA_ERR_WORKSPACE;
   if (pk) {
     stage_geom<T>(s, sys_t<T>(s).vals, &w.geom);
@@ -2098,8 +2049,7 @@ int refine_solve(const gfea_system* s, const double* b, double* x, const gfea_pc
   Scal hs;
   GFEA_CUDA_TRY(cudaMemsetAsync(w.sc, 0, sizeof(Scal), st));
   GFEA_CUDA_TRY(cudaMemsetAsync(w.flag, 0, sizeof(int32_t) * 4, st));
-  int e = launch_bjacobi<T>(s, w, st);
-  if (e) return e;
+  int e = GFEA_OK;
   int G = pick_lanes(s, o->lanes, vt);
   if (w.coarse) {
     const bool dbg = !direct_only && getenv("GFEA_DEBUG") != nullptr;
@@ -2121,6 +2071,39 @@ int refine_solve(const gfea_system* s, const double* b, double* x, const gfea_pc
       for (int i = 0; i < 3; ++i) cudaEventDestroy(ev[i]);
     }
   }
+  ResidentGeom geom;
+  if (use_resident<T>(s, o, w, direct_only, &geom)) {
+    // pa and pb are adjacent: the packets of p; rcp holds three accumulators
+    // and, behind them, the packets of ec
+    ResidentProblem<T> P{};
+    P.S = sys_t<T>(s);
+    P.vals64 = s->vals64;
+    P.b = b;
+    P.x = x;
+    P.p = (T*)w.pa;
+    P.C = w.C;
+    P.ec = w.coarse ? reinterpret_cast<T*>(w.C.rcp + 4 * (size_t)w.C.nc) : nullptr;
+    P.coarse = w.coarse ? 1 : 0;
+    P.box = reinterpret_cast<double*>(w.box);
+    P.out = reinterpret_cast<gfea_pcg_result*>(w.sc);
+    P.rtol = o->rtol;
+    P.delta2 = delta2;
+    P.max_iters = o->max_iters;
+    P.max_upd = o->max_refine > 0 ? o->max_refine : 200;
+    GFEA_CUDA_TRY(cudaMemsetAsync(P.box, 0, kResidentBox / (kSMs * kSMs) * geom.grid * geom.grid, st));
+    e = resident_launch<T>(s->dof_n, P, geom, st);
+    if (e) return e;
+    GFEA_CUDA_TRY(cudaMemcpyAsync(res, P.out, sizeof(*res), cudaMemcpyDeviceToHost, st));
+    GFEA_CUDA_TRY(cudaStreamSynchronize(st));
+    if (getenv("GFEA_DEBUG"))
+      fprintf(stderr, "[gfea pcg%d] resident: %d CTAs, iterations %d, updates %d, status %d, rel residual %.3e, %.2f ms\n",
+              fp64 ? 64 : 32, geom.grid, res->iterations, res->refinements, res->status,
+              res->rel_residual,
+              std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t_start).count());
+    return res->status;
+  }
+  e = launch_bjacobi<T>(s, w, st);
+  if (e) return e;
   e = launch_resid(s, G, b, x, w, true, st);
   if (e) return e;
   int32_t flag = 0;
@@ -2294,10 +2277,12 @@ extern "C" int gfea_tune_spmv(const gfea_system* s, int value_type, const void* 
 extern "C" int gfea_pcg_workspace_size(const gfea_system* s, const gfea_pcg_opts* o, size_t* bytes) {
   if (!s || !o || !bytes || s->n_nodes <= 0 || s->dof_n < 1 || s->dof_n > 3) return GFEA_ERR_ARG;
   const int target = coarse_target(s, o);
+  const size_t pk = o->precision == GFEA_F64 ? packed_bytes<double>(s, true) : packed_bytes<float>(s, true);
+  const size_t box = pk ? 0 : kResidentBox;  // staged tiles or the resident solve's packets
   if (o->precision == GFEA_F64)
-    *bytes = pcg_layout<double>(s->n_nodes, s->dof_n, target, nullptr, nullptr, packed_bytes<double>(s, true));
+    *bytes = pcg_layout<double>(s->n_nodes, s->dof_n, target, nullptr, nullptr, pk, box);
   else
-    *bytes = pcg_layout<float>(s->n_nodes, s->dof_n, target, nullptr, nullptr, packed_bytes<float>(s, true));
+    *bytes = pcg_layout<float>(s->n_nodes, s->dof_n, target, nullptr, nullptr, pk, box);
   return GFEA_OK;
 }
 
