@@ -35,6 +35,8 @@
 
 #include "coarse.cuh"
 #include "common.cuh"
+#include "ff.cuh"
+#include "inverse.cuh"
 #include "pcg_types.cuh"
 #include "resident.cuh"
 #include "rowops.cuh"
@@ -496,7 +498,7 @@ __global__ void coarse_assemble_kernel(SysT<T> S, CoarseDev C) {
 
 // Unit diagonal for empty or fully constrained coarse DOFs, a 1e-10 relative
 // shift elsewhere (rotation modes of degenerate aggregates), identity in inv.
-// (zero_tol, shift): (1e-14, 1e-10) for a coarse matrix built in FP64,
+// (zero_tol, shift) of a batch's matrices: (1e-14, 1e-10) for those built in FP64,
 // (1e-6, 1e-6) for one built from FP32 values, whose rounding can reach the
 // 1e-6 level in nearly degenerate modes.
 __device__ __forceinline__ void coarse_regularize_body(const CoarseDev& C, double zero_tol, double shift) {
@@ -516,12 +518,8 @@ __device__ __forceinline__ void coarse_regularize_body(const CoarseDev& C, doubl
   }
 }
 
-__global__ void coarse_regularize_kernel(CoarseDev C, double zero_tol, double shift) {
-  coarse_regularize_body(C, zero_tol, shift);
-}
-
-// In-place blocked Gauss-Jordan inversion of the SPD coarse matrix (no
-// pivoting: every pivot block of an SPD matrix is SPD).  For the pivot block
+// In-place blocked Gauss-Jordan inversion of a batch's SPD coarse matrices (a
+// single system's: inverse.cu; no pivoting: every pivot block of an SPD matrix is SPD).  For the pivot block
 // K = [k0, k0 + b) of A = [[A11, A12], [A21, A22]]:
 //   A11 <- A11^-1,  A12 <- A11^-1 A12,  A21 <- -A21 A11^-1,
 //   A22 <- A22 - A21 A11^-1 A12,
@@ -529,46 +527,6 @@ __global__ void coarse_regularize_kernel(CoarseDev C, double zero_tol, double sh
 // the old column panel A*1 (colp) and A11^-1 (pinv); gj_update applies the
 // rank-b update to every element (each read and written by one thread).
 constexpr int kGJB = 16;
-
-// Float-float arithmetic of the inversion's trailing updates: a value is an
-// unevaluated pair hi + lo of floats (~2^-44 relative), products by the exact
-// FMA split, sums by TwoSum (Knuth); GB300 runs FP32 at 64x its FP64 rate, so
-// the n^3 update FMAs cost less than in FP64 even at ~12 FP32 operations each.
-__device__ __forceinline__ void ff_split(double d, float& hi, float& lo) {
-  hi = (float)d;
-  lo = (float)(d - (double)hi);
-}
-
-// (sh, sl) += (ah, al) (bh, bl); the al bl term is below the pair's precision
-__device__ __forceinline__ void ff_fma_acc(float& sh, float& sl, float ah, float al, float bh, float bl) {
-  const float p = ah * bh;
-  const float e = fmaf(ah, bh, -p) + fmaf(ah, bl, al * bh);
-  const float t = sh + p;
-  const float bp = t - sh;
-  sl += ((sh - (t - bp)) + (p - bp)) + e;
-  sh = t;
-}
-
-// (ah, al) - (sh, sl), normalised
-__device__ __forceinline__ void ff_sub(float ah, float al, float sh, float sl, float& hi, float& lo) {
-  const float t = ah - sh;
-  const float bp = t - ah;
-  const float err = (ah - (t - bp)) + (-sh - bp);
-  const float l = err + (al - sl);
-  hi = t + l;
-  lo = l - (hi - t);
-}
-
-__global__ void ff_split_kernel(const double* __restrict__ a, float* __restrict__ hi, float* __restrict__ lo, int64_t n) {
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
-    ff_split(a[i], hi[i], lo[i]);
-}
-
-__global__ void ff_merge_kernel(double* __restrict__ a, const float* __restrict__ hi, const float* __restrict__ lo,
-                                int64_t n) {
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
-    a[i] = (double)hi[i] + (double)lo[i];
-}
 
 // block (bx, l): row l of the transformed row panel for columns bx * 128 ..;
 // every block inverts the b x b pivot block itself (b steps in shared
@@ -613,10 +571,6 @@ __device__ __forceinline__ void gj_panel_body(const CoarseDev& C, int k0, int b,
   }
 }
 
-__global__ void __launch_bounds__(128) gj_panel_kernel(CoarseDev C, int k0, int b) {
-  gj_panel_body(C, k0, b, blockIdx.x, blockIdx.y);
-}
-
 // Block (bx, by) owns column j = bx * blockDim + tid and rows by, by + gridDim.y, ...
 __device__ __forceinline__ void gj_update_body(const CoarseDev& C, int k0, int b, int bx, int by, int gy) {
   const int n = C.nc;
@@ -648,10 +602,6 @@ __device__ __forceinline__ void gj_update_body(const CoarseDev& C, int k0, int b
     C.Ahi[q] = vh;
     C.Alo[q] = vl;
   }
-}
-
-__global__ void __launch_bounds__(128) gj_update_kernel(CoarseDev C, int k0, int b) {
-  gj_update_body(C, k0, b, blockIdx.x, blockIdx.y, gridDim.y);
 }
 
 // x, r update (mode 0) and restriction rc += R_a^T r_a.  The node loop runs
@@ -1666,27 +1616,13 @@ int coarse_matrix(const gfea_system* s, CoarseDev& C, cudaStream_t st, cudaEvent
   const SysT<T> S = sys_t<T>(s);
   GFEA_D_SWITCH(D, (coarse_assemble_kernel<DD, T><<<grid_elems(Nn), kThreads, 0, st>>>(S, C)));
   GFEA_LAUNCH_CHECK();
-  if (sizeof(T) == 4)
-    coarse_regularize_kernel<<<1, 256, 0, st>>>(C, 1e-6, 1e-6);
-  else
-    coarse_regularize_kernel<<<1, 256, 0, st>>>(C, 1e-14, 1e-10);
-  GFEA_LAUNCH_CHECK();
   if (mark) GFEA_CUDA_TRY(cudaEventRecord(mark, st));
-  const int64_t n2 = (int64_t)C.nc * C.nc;
-  ff_split_kernel<<<grid_elems(n2), kThreads, 0, st>>>(C.Ac, C.Ahi, C.Alo, n2);
-  GFEA_LAUNCH_CHECK();
-  const int gx = (int)ceil_div(C.nc, 128);
-  const int gy = (int)std::min<int64_t>(C.nc, ceil_div(2 * kMaxBlocks, gx));
-  for (int k0 = 0; k0 < C.nc; k0 += kGJB) {
-    const int b = std::min(kGJB, C.nc - k0);
-    gj_panel_kernel<<<dim3(gx, b), 128, 0, st>>>(C, k0, b);
-    GFEA_LAUNCH_CHECK();
-    gj_update_kernel<<<dim3(gx, gy), 128, 0, st>>>(C, k0, b);
-    GFEA_LAUNCH_CHECK();
-  }
-  ff_merge_kernel<<<grid_elems(n2), kThreads, 0, st>>>(C.Ac, C.Ahi, C.Alo, n2);
-  GFEA_LAUNCH_CHECK();
-  return GFEA_OK;
+  // FP64 values: the shift keeps nearly degenerate modes (rotations of one-
+  // or two-node aggregates) well above the float-float rounding of the
+  // inversion (~1e-12 of the largest entry): at 1e-10 the 384-unknown coarse
+  // matrix of a 64-aggregate HEXA8 bar came out indefinite; iterations are the
+  // same with either.
+  return sizeof(T) == 4 ? coarse_inverse(C, 1e-6, 1e-6, st) : coarse_inverse(C, 1e-14, 1e-8, st);
 }
 
 template <typename T>
