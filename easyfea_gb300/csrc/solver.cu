@@ -431,63 +431,79 @@ __global__ void aggregate_kernel(const double* __restrict__ coord, int64_t Nn, d
   }
 }
 
-// A_c += R_a^T K_ab R_b, summed per node over neighbours sharing an aggregate
-// (T: the iteration's value type -- the FP32 operator of the mixed path gives
-// a coarse matrix accurate to ~1e-6, plenty for a preconditioner, on the FP32
-// pipe; sums go to A_c in FP64).
+// A_c += R_a^T K_ab R_b (T: the iteration's value type -- the FP32 operator of
+// the mixed path gives a coarse matrix accurate to ~1e-6, plenty for a
+// preconditioner, on the FP32 pipe; sums go to A_c in FP64).
+//
+// A thread per node a and mode m: it takes the neighbours' aggregates in
+// ascending order, sums y = sum_b K_ab R_b[:, m] over the neighbours of one
+// aggregate (a column of R_b has one or two entries) and adds R_a^T y to the
+// coarse columns of that aggregate: D products per pair instead of the full
+// D x nr and nr x nr ones, and no per-thread table of aggregates (the local
+// memory of the thread-per-node form it replaces, 0.40 ms for 13,104 HEXA8
+// nodes in FP64 and 1.40 ms for 689,000 in FP32).
 template <int D, typename T>
 __device__ __forceinline__ void coarse_assemble_body(const SysT<T>& S, const CoarseDev& C, int64_t bx, int64_t gx) {
   constexpr int nr = Modes<D>::nr;
-  constexpr int kSlots = 8;
-  for (int64_t a = bx * (int64_t)blockDim.x + threadIdx.x; a < S.Nn; a += gx * blockDim.x) {
+  for (int64_t t = bx * (int64_t)blockDim.x + threadIdx.x; t < S.Nn * nr; t += gx * blockDim.x) {
+    const int64_t a = t / nr;
+    const int m = (int)(t - a * nr);
     const int ga = C.agg[a];
     T Ra[D][nr];
     node_modes<D, T>(C.off[a], S.known + a * D, Ra);
-    int sid[kSlots];
-    T acc[kSlots][nr][nr];
-    int ns = 0;
     const int32_t p0 = S.node_ptr[a], nb = S.node_ptr[a + 1] - p0;
     const int32_t W = D * nb;
-    for (int k = 0; k < nb; ++k) {
-      const int32_t b = S.nbr[p0 + k];
-      const int gb = C.agg[b];
-      T Rb[D][nr];
-      node_modes<D, T>(C.off[b], S.known + (int64_t)b * D, Rb);
-      // K_ab R_b (D x nr)
-      T KR[D][nr];
-      for (int i = 0; i < D; ++i)
-        for (int m = 0; m < nr; ++m) {
-          T v = 0;
-          for (int j = 0; j < D; ++j) v += S.vals[(int64_t)D * D * p0 + (int64_t)i * W + D * k + j] * Rb[j][m];
-          KR[i][m] = v;
+    const int32_t* __restrict__ nbr = S.nbr + p0;
+    const T* __restrict__ rows = S.vals + (int64_t)D * D * p0;
+    // the column's components: j1 with coefficient 1 (translations), or j1
+    // and j2 with the offsets along the other axes (rotations)
+    const bool rot = m >= D;
+    const int ax = m - D;  // 2D: the one rotation (x, y); 3D: rotation about axis ax
+    const int j1 = !rot ? m : (D == 2 ? 1 : (ax == 0 ? 2 : (ax == 1 ? 0 : 1)));
+    const int j2 = !rot ? m : (D == 2 ? 0 : (ax == 0 ? 1 : (ax == 1 ? 2 : 0)));
+    int next = INT32_MAX;
+    for (int k = 0; k < nb; ++k) next = min(next, __ldg(C.agg + __ldg(nbr + k)));
+    while (next != INT32_MAX) {
+      const int cur = next;
+      next = INT32_MAX;
+      T y[D];
+#pragma unroll
+      for (int i = 0; i < D; ++i) y[i] = 0;
+      for (int k = 0; k < nb; ++k) {
+        const int64_t b = __ldg(nbr + k);
+        const int g = __ldg(C.agg + b);
+        if (g > cur) next = min(next, g);
+        if (g != cur) continue;
+        T c1 = 1, c2 = 0;
+        if constexpr (D > 1) {
+          if (rot) {
+            const float4 o = __ldg(C.off + b);
+            if (D == 2) {
+              c1 = o.x;
+              c2 = -o.y;
+            } else {
+              c1 = ax == 0 ? o.y : (ax == 1 ? o.z : o.x);
+              c2 = -(ax == 0 ? o.z : (ax == 1 ? o.x : o.y));
+            }
+          }
         }
-      int slot = -1;
-      for (int q = 0; q < ns; ++q)
-        if (sid[q] == gb) slot = q;
-      if (slot < 0) {
-        if (ns == kSlots) {  // flush (rare: more distinct neighbour aggregates than slots)
-          for (int q = 0; q < ns; ++q)
-            for (int m = 0; m < nr; ++m)
-              for (int l = 0; l < nr; ++l)
-                atomicAdd(&C.Ac[(int64_t)(ga * nr + m) * C.nc + sid[q] * nr + l], (double)acc[q][m][l]);
-          ns = 0;
+        if (S.known[b * D + j1]) c1 = 0;
+        if (rot && S.known[b * D + j2]) c2 = 0;
+#pragma unroll
+        for (int i = 0; i < D; ++i) {
+          const T* row = rows + (int64_t)i * W + D * k;
+          y[i] += __ldg(row + j1) * c1;
+          if (rot) y[i] += __ldg(row + j2) * c2;
         }
-        slot = ns++;
-        sid[slot] = gb;
-        for (int m = 0; m < nr; ++m)
-          for (int l = 0; l < nr; ++l) acc[slot][m][l] = 0;
       }
-      for (int m = 0; m < nr; ++m)
-        for (int l = 0; l < nr; ++l) {
-          T v = 0;
-          for (int i = 0; i < D; ++i) v += Ra[i][m] * KR[i][l];
-          acc[slot][m][l] += v;
-        }
+#pragma unroll
+      for (int l = 0; l < nr; ++l) {
+        T v = 0;
+#pragma unroll
+        for (int i = 0; i < D; ++i) v += Ra[i][l] * y[i];
+        if (v != 0) atomicAdd(&C.Ac[(int64_t)(ga * nr + l) * C.nc + cur * nr + m], (double)v);
+      }
     }
-    for (int q = 0; q < ns; ++q)
-      for (int m = 0; m < nr; ++m)
-        for (int l = 0; l < nr; ++l)
-          atomicAdd(&C.Ac[(int64_t)(ga * nr + m) * C.nc + sid[q] * nr + l], (double)acc[q][m][l]);
   }
 }
 
@@ -1614,7 +1630,7 @@ int coarse_matrix(const gfea_system* s, CoarseDev& C, cudaStream_t st, cudaEvent
   const int D = s->dof_n;
   GFEA_CUDA_TRY(cudaMemsetAsync(C.Ac, 0, sizeof(double) * C.nc * C.nc, st));
   const SysT<T> S = sys_t<T>(s);
-  GFEA_D_SWITCH(D, (coarse_assemble_kernel<DD, T><<<grid_elems(Nn), kThreads, 0, st>>>(S, C)));
+  GFEA_D_SWITCH(D, (coarse_assemble_kernel<DD, T><<<grid_elems(Nn * coarse_nr(D)), kThreads, 0, st>>>(S, C)));
   GFEA_LAUNCH_CHECK();
   if (mark) GFEA_CUDA_TRY(cudaEventRecord(mark, st));
   // FP64 values: the shift keeps nearly degenerate modes (rotations of one-

@@ -67,3 +67,57 @@ def test_inverse_of_the_coarse_matrix(target, precision):
     tol = cond * (2.0**-40 if precision == 0 else 2.0**-20)
     assert np.abs(inv @ Ac - np.eye(nc)).max() <= tol
     assert np.abs(inv - inv.T).max() <= tol * np.abs(inv).max()
+
+
+@pytest.mark.parametrize("elem,counts", [("QUAD4", (23, 7)), ("TRI6", (9, 5)), ("HEXA8", (11, 4, 3)), ("TETRA4", (7, 3, 3))])
+@pytest.mark.parametrize("target", [1, 5, 9])
+def test_rigid_body_modes_of_an_elastic_operator(elem, counts, target):
+    """A_c = R^T K R with translations and rotations of every aggregate, known
+    DOFs masked: neighbours in several aggregates, whole aggregates inside."""
+    import torch
+
+    from easyfea_gb300 import Models, _lib
+    from easyfea_gb300 import mesh as gmesh
+    from easyfea_gb300 import simulations as Simulations
+
+    dim = len(counts)
+    make = gmesh.Mesh_Rect if dim == 2 else gmesh.Mesh_Box
+    m = make(gmesh.ElemType(elem), *((30.0, 8.0, 6.0)[:dim]), *counts)
+    simu = Simulations.Elastic(m, Models.Elastic.Isotropic(dim, E=210000.0, v=0.3, planeStress=dim == 2))
+    op = simu.K_device
+    known = np.zeros(m.Nn * dim, np.uint8)
+    left = m.Nodes_Conditions(lambda x, y, z: x == 0)
+    for k in range(dim):
+        known[left * dim + k] = 1
+    known[5] = 1
+    kd = torch.as_tensor(known, device="cuda")
+    s = op.system(kd)
+    o = _lib.PcgOpts(_lib.ABI_VERSION, _lib.F64, 0, 0, 0.0, 0.0, 0, 0, target, 0)
+    L = _lib.load()
+    nb = ctypes.c_size_t()
+    _lib.check(L.gfea_coarse_workspace_size(ctypes.byref(s), ctypes.byref(o), ctypes.byref(nb)), "size")
+    work = torch.empty(nb.value, dtype=torch.uint8, device="cuda")
+    lv = _lib.CoarseLevel()
+    _lib.check(L.gfea_coarse_setup(ctypes.byref(s), ctypes.byref(o), 0, _lib.ptr(work), work.numel(),
+                                   ctypes.byref(lv), _lib.stream()), "setup")
+    torch.cuda.synchronize()
+
+    def read(ptr, n, dtype):
+        off = ptr - work.data_ptr()
+        return work[off:off + n * np.dtype(dtype).itemsize].cpu().numpy().view(dtype)
+
+    agg = read(lv.agg, m.Nn, np.int32)
+    off = read(lv.off, 4 * m.Nn, np.float32).reshape(-1, 4).astype(np.float64)
+    nc, nr = lv.nc, lv.nr
+    R = np.zeros((m.Nn * dim, nc))
+    for a in range(m.Nn):
+        x, y, z = off[a, :3]
+        modes = (np.array([[1, 0, -y], [0, 1, x]]) if dim == 2 else
+                 np.array([[1, 0, 0, 0, z, -y], [0, 1, 0, -z, 0, x], [0, 0, 1, y, -x, 0]]))
+        R[a * dim:(a + 1) * dim, agg[a] * nr:(agg[a] + 1) * nr] = modes
+    R[known.astype(bool)] = 0
+    Ac = R.T @ (op.to_scipy() @ R)
+    d = np.diag(Ac).copy()
+    np.fill_diagonal(Ac, np.where(d > 1e-14 * d.max(), d + 1e-8 * d.max(), d.max()))
+    inv = read(lv.inv, nc * nc, np.float64).reshape(nc, nc)
+    assert np.abs(inv @ Ac - np.eye(nc)).max() <= np.linalg.cond(Ac) * 2.0**-40
