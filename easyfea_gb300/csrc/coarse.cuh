@@ -42,4 +42,19 @@ __device__ __forceinline__ void node_modes(float4 o, const uint8_t* kn, T (&R)[D
   }
 }
 
+// Component k of R e at a node of offset o (unmasked; e: the coefficients of
+// its aggregate's modes).
+template <int D, typename T>
+__device__ __forceinline__ T mode_row(int k, float4 o, const T* __restrict__ e) {
+  if constexpr (D == 1) {
+    return e[0];
+  } else if constexpr (D == 2) {
+    return k == 0 ? e[0] - (T)o.y * e[2] : e[1] + (T)o.x * e[2];
+  } else {
+    return k == 0   ? e[0] + ((T)o.z * e[4] - (T)o.y * e[5])
+           : k == 1 ? e[1] + ((T)o.x * e[5] - (T)o.z * e[3])
+                    : e[2] + ((T)o.y * e[3] - (T)o.x * e[4]);
+  }
+}
+
 }  // namespace gfea

@@ -11,12 +11,15 @@
 // operator P A P + (I - P) (P = diag(unknown)); search directions vanish on
 // known DOFs, so the product is a plain SpMV with known rows zeroed.
 //
-// One PCG iteration is three kernels (block-Jacobi) or five (two-level):
-//   dir      : p' = z + beta p
-//   apply    : Ap' (masked SpMV), p'.Ap', alpha
-//   update   : x += alpha p', r -= alpha Ap', z = D^-1 r, r.z, r.r, beta
-// with the coarse level, update is split into update_r (x, r, restriction),
-// coarse_gemv and finish_z (z = D^-1 r + prolonged correction, dots, beta).
+// One PCG iteration with block-Jacobi alone is three kernels:
+//   dir       : p' = z + beta p
+//   apply     : Ap' (masked SpMV), p'.Ap', alpha
+//   update    : x += alpha p', r -= alpha Ap', z = D^-1 r, r.z, r.r, beta
+// and with the coarse level four (five with restriction copies):
+//   apply     : Ap, p.Ap, alpha
+//   update_r  : x += alpha p, r -= alpha Ap, y = D^-1 r, r.y, r.r, rc = R^T r
+//   gemv      : ec = A_c^-1 rc, r.z = r.y + rc.ec, beta
+//   direction : p = y + R ec + beta p
 // Reductions are per-block partials summed in a fixed order by the last block
 // to finish (atomic ticket, no spinning), which also derives the scalar
 // recurrences (alpha, beta, convergence) on the device.  Kernels return early
@@ -50,7 +53,7 @@ constexpr int kThreads = 256;
 constexpr int kMaxBlocks = kSMs * 8;
 
 struct Scal {
-  double rz, rr, pap, alpha, beta, bb, tol2, rr_true, absAx;
+  double rz, rr, pap, alpha, beta, bb, tol2, rr_true, absAx, ry;
   int32_t done, iters, status, max_iters;
   uint32_t ticket1, ticket2, ticket3, pad;
 };
@@ -59,9 +62,8 @@ struct Scal {
 // kernel kind; gfea_profile_read returns the SpMV kernel's (the dominant
 // launch of a solve).  Events are recorded after each launch of a chunk of
 // iterations and attributed once the chunk's performed iterations are known.
-enum ProfTag { kTagDir, kTagApply, kTagUpdate, kTagRestrict, kTagGemv, kTagFinish, kNumTags };
-const char* const kTagNames[kNumTags] = {"direction", "spmv", "update", "update+restrict", "coarse gemv",
-                                         "finish z"};
+enum ProfTag { kTagDir, kTagApply, kTagUpdate, kTagRestrict, kTagGemv, kNumTags };
+const char* const kTagNames[kNumTags] = {"direction", "spmv", "update", "update+restrict", "coarse gemv"};
 
 // Solves may run concurrently from several host threads (one stream each):
 // the events of a chunk are per thread, the totals are shared under a mutex.
@@ -263,6 +265,82 @@ __global__ void __launch_bounds__(kThreads) resid_kernel(SysT<T> S, const float*
       r[dof] = ri;
       v[0] += ri * ri;
       v[1] += rci * rci;
+      v[2] += ai * ai;
+    }
+  }
+  double out[3];
+  if (reduce_last<3>(v, partials, &sc->ticket3, out) && threadIdx.x == 0) {
+    sc->rr_true = out[0];
+    if (KN) sc->bb = out[1];
+    sc->absAx = out[2];
+  }
+}
+
+// resid_kernel with lane D n + j owning component j of node n of a warp's
+// 32 / D nodes (as in the staged SpMV): FP64 instructions bound the residual,
+// and a lane group that shares a row spends as many of them on adding its
+// lanes up as on the products (about 16 a node in 3D, 9 here).  The values a
+// warp reads are strided; blocks take contiguous nodes and only three run per
+// SM, so that a line is used up while it is in L1.
+template <int D, bool KN, bool AB32>
+__global__ void __launch_bounds__(kThreads, 3) resid_comp_kernel(SysT<double> S, const float* __restrict__ v32,
+                                                                 const float* __restrict__ x32,
+                                                                 const double* __restrict__ b,
+                                                                 const double* __restrict__ x, double* __restrict__ r,
+                                                                 double* partials, Scal* sc) {
+  constexpr int NPW = 32 / D;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int64_t tiles = ceil_div(S.Nn, NPW), per = ceil_div(tiles, gridDim.x);
+  const int64_t t1 = min((int64_t)(blockIdx.x + 1) * per, tiles);
+  double v[3] = {0, 0, 0};
+  for (int64_t t = blockIdx.x * per + warp; t < t1; t += kThreads / 32) {
+    const int64_t a = t * NPW + lane / D;
+    const bool live = lane < NPW * D && a < S.Nn;
+    const int j = live ? lane % D : 0;
+    double all[D], kn[D], ab[D];
+    float ab32[D];
+#pragma unroll
+    for (int i = 0; i < D; ++i) {
+      all[i] = kn[i] = ab[i] = 0;
+      ab32[i] = 0.f;
+    }
+    if (live) {
+      const int32_t p0 = S.node_ptr[a], nb = S.node_ptr[a + 1] - p0;
+      const int32_t W = D * nb;
+      const double* base = S.vals + (int64_t)D * D * p0 + j;
+      const float* base32 = AB32 ? v32 + (int64_t)D * D * p0 + j : nullptr;
+#pragma unroll 3
+      for (int32_t k = 0; k < nb; ++k) {
+        const int64_t col = (int64_t)__ldg(S.nbr + p0 + k) * D + j;
+        const double xv = __ldg(x + col);
+        const bool isk = KN && S.known[col];
+        const float xa32 = AB32 ? fabsf(__ldg(x32 + col)) : 0.f;
+#pragma unroll
+        for (int i = 0; i < D; ++i) {
+          const double w = __ldg(base + (int64_t)i * W + D * k);
+          all[i] += w * xv;
+          if (isk) kn[i] += w * xv;
+          if (AB32)
+            ab32[i] += fabsf(__ldg(base32 + (int64_t)i * W + D * k)) * xa32;
+          else
+            ab[i] += fabs(w) * fabs(xv);
+        }
+      }
+    }
+    const int el = live ? lane : lane - lane % D;
+    const double s_all = node_rows_exchange<D, double>(all, j, el);
+    const double s_kn = KN ? node_rows_exchange<D, double>(kn, j, el) : 0.0;
+    const double s_ab = AB32 ? (double)node_rows_exchange<D, float>(ab32, j, el) : node_rows_exchange<D, double>(ab, j, el);
+    if (live) {
+      const int64_t dof = a * D + j;
+      const bool unk = !S.known[dof];
+      const double bv = b[dof];
+      const double ri = unk ? bv - s_all : 0.0;
+      const double rci = unk ? bv - s_kn : 0.0;
+      const double ai = unk ? s_ab + fabs(bv) : 0.0;
+      r[dof] = ri;
+      v[0] += ri * ri;
+      if (KN) v[1] += rci * rci;
       v[2] += ai * ai;
     }
   }
@@ -620,18 +698,26 @@ __device__ __forceinline__ void gj_update_body(const CoarseDev& C, int k0, int b
   }
 }
 
-// x, r update (mode 0) and restriction rc += R_a^T r_a.  The node loop runs
-// whole warps (stride a multiple of 32) for the warp-level pre-reduction.
+// x, r update (mode 0), y = D^-1 r, restriction rc += R_a^T r_a and the sums
+// r.y, r.r.  The node loop runs whole warps (stride a multiple of 32) for the
+// warp-level pre-reduction.
+//
+// With z = y + R ec, r.z = r.y + rc.ec: beta is known once the coarse solve
+// is, so z is never stored and one kernel (direction_kernel) forms p from y,
+// ec and the old p, where a kernel of its own formed z and its dots (25 us
+// for the 2.02M-unknown box in FP32) and another p (9 us).
 template <int D, typename T>
 __global__ void __launch_bounds__(kThreads) update_r_kernel(int64_t Nn, const uint8_t* __restrict__ known,
-                                                            T* __restrict__ x,
-                                                            T* __restrict__ r, const T* __restrict__ p,
-                                                            const T* __restrict__ Ap, Scal* sc, CoarseDev C,
-                                                            int mode) {
+                                                            const T* __restrict__ dinv, T* __restrict__ x,
+                                                            T* __restrict__ r, T* __restrict__ y,
+                                                            const T* __restrict__ p, const T* __restrict__ Ap,
+                                                            double* partials, Scal* sc, CoarseDev C, int mode) {
   if (mode == 0 && sc->done) return;
   constexpr int nr = Modes<D>::nr;
-  const double alpha = mode == 0 ? sc->alpha : 0.0;
+  const T alpha = mode == 0 ? (T)sc->alpha : (T)0;
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
+  double* rc = C.ncopies > 1 ? C.rcp + (int64_t)(blockIdx.x % kRcCopies) * C.nc : C.rc;
+  DotAcc<T> ry, rr;
   for (int64_t a = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; a - (threadIdx.x & 31) < Nn; a += stride) {
     T v[nr];
 #pragma unroll
@@ -644,11 +730,21 @@ __global__ void __launch_bounds__(kThreads) update_r_kernel(int64_t Nn, const ui
         const int64_t dof = a * D + i;
         T ri = r[dof];
         if (mode == 0) {
-          x[dof] += (T)alpha * p[dof];
-          ri -= (T)alpha * Ap[dof];
+          x[dof] += alpha * p[dof];
+          ri -= alpha * Ap[dof];
           r[dof] = ri;
         }
         rl[i] = ri;
+      }
+#pragma unroll
+      for (int i = 0; i < D; ++i) {
+        T yi = 0;
+#pragma unroll
+        for (int j = 0; j < D; ++j) yi += dinv[a * D * D + i * D + j] * rl[j];
+        if (known[a * D + i]) yi = 0;
+        y[a * D + i] = yi;
+        ry.add_prod(rl[i], yi);
+        rr.add_prod(rl[i], rl[i]);
       }
       g = C.agg[a];
       T R[D][nr];
@@ -658,7 +754,13 @@ __global__ void __launch_bounds__(kThreads) update_r_kernel(int64_t Nn, const ui
 #pragma unroll
         for (int i = 0; i < D; ++i) v[m] += R[i][m] * rl[i];
     }
-    restrict_add<nr, T>(C.ncopies > 1 ? C.rcp + (int64_t)(blockIdx.x % kRcCopies) * C.nc : C.rc, g, v);
+    restrict_add<nr, T>(rc, g, v);
+  }
+  const DotAcc<T> v[2] = {ry, rr};
+  double out[2];
+  if (reduce_last_acc<2, T>(v, partials, &sc->ticket2, out) && threadIdx.x == 0) {
+    sc->ry = out[0];
+    sc->rr = out[1];
   }
 }
 
@@ -682,9 +784,13 @@ __global__ void __launch_bounds__(kThreads) rc_sum_kernel(CoarseDev C, const Sca
 // flight to stream the L2-resident inverse), fixed-order block reduction.
 constexpr int kGemvThreads = 128;
 
-__global__ void __launch_bounds__(kGemvThreads) coarse_gemv_kernel(CoarseDev C, const Scal* sc, int mode) {
+// The last block to finish completes r.z = r.y + rc.ec, derives beta and the
+// convergence state exactly as update_kernel does, and clears a single-copy
+// rc for the next restriction.
+__global__ void __launch_bounds__(kGemvThreads) coarse_gemv_kernel(CoarseDev C, double* partials, Scal* sc, int mode) {
   if (mode == 0 && sc->done) return;
   __shared__ double sh[kGemvThreads / 32];
+  double dot[1] = {0};
   for (int i = blockIdx.x; i < C.nc; i += gridDim.x) {
     const double* row = C.Ac + (int64_t)i * C.nc;
     double v = 0;
@@ -699,54 +805,18 @@ __global__ void __launch_bounds__(kGemvThreads) coarse_gemv_kernel(CoarseDev C, 
       for (int w = 0; w < kGemvThreads / 32; ++w) t += sh[w];
       C.ec[i] = t;
       C.ecf[i] = (float)t;
+      dot[0] += t * C.rc[i];
     }
     __syncthreads();
   }
-}
-
-// z = D^-1 r + R_a ec (masked), partial r.z and r.r, rc reset; the last block
-// derives beta and the convergence state exactly as update_kernel does.
-template <int D, typename T>
-__global__ void __launch_bounds__(kThreads) finish_z_kernel(int64_t Nn, const uint8_t* __restrict__ known,
-                                                            const T* __restrict__ dinv, const T* __restrict__ r,
-                                                            T* __restrict__ z, double* partials, Scal* sc,
-                                                            CoarseDev C, int mode) {
-  if (mode == 0 && sc->done) return;
-  constexpr int nr = Modes<D>::nr;
-  DotAcc<T> rz, rr;
-  const T* ec = sizeof(T) == 4 ? (const T*)C.ecf : (const T*)C.ec;
-  for (int64_t a = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; a < Nn; a += (int64_t)gridDim.x * blockDim.x) {
-    T rl[D];
-#pragma unroll
-    for (int i = 0; i < D; ++i) rl[i] = r[a * D + i];
-    const int g = C.agg[a];
-    T R[D][nr];
-    node_modes<D, T>(C.off[a], known + a * D, R);
-    T e[nr];
-#pragma unroll
-    for (int m = 0; m < nr; ++m) e[m] = ec[g * nr + m];
-#pragma unroll
-    for (int i = 0; i < D; ++i) {
-      T zi = 0;
-#pragma unroll
-      for (int j = 0; j < D; ++j) zi += dinv[a * D * D + i * D + j] * rl[j];
-#pragma unroll
-      for (int m = 0; m < nr; ++m) zi += R[i][m] * e[m];
-      if (known[a * D + i]) zi = 0;
-      z[a * D + i] = zi;
-      rz.add_prod(rl[i], zi);
-      rr.add_prod(rl[i], rl[i]);
-    }
-  }
-  if (C.ncopies == 1)  // single copy: clear rc (read by this iteration's GEMV) for the next restriction
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < C.nc; i += gridDim.x * blockDim.x) C.rc[i] = 0;
-  const DotAcc<T> v[2] = {rz, rr};
-  double out[2];
-  if (reduce_last_acc<2, T>(v, partials, &sc->ticket2, out) && threadIdx.x == 0) {
-    const double rz_new = out[0], rr = out[1];
+  double out[1];
+  if (!reduce_last<1>(dot, partials, &sc->ticket1, out)) return;
+  if (C.ncopies == 1)
+    for (int i = threadIdx.x; i < C.nc; i += blockDim.x) C.rc[i] = 0;
+  if (threadIdx.x == 0) {
+    const double rz_new = sc->ry + out[0], rr = sc->rr;
     sc->beta = next_beta(mode, rz_new, sc->rz, sc->beta);
     sc->rz = rz_new;
-    sc->rr = rr;
     if (mode != 0) return;
     sc->iters += 1;
     if (!isfinite(rr) || !isfinite(rz_new)) {
@@ -759,6 +829,24 @@ __global__ void __launch_bounds__(kThreads) finish_z_kernel(int64_t Nn, const ui
       sc->status = GFEA_ERR_NOT_CONVERGED;
       sc->done = 1;
     }
+  }
+}
+
+// p = z + beta p with z = y + R_a ec (masked): a thread per unknown.  The
+// iteration that converged keeps its p (a reliable update continues from it).
+template <int D, typename T>
+__global__ void __launch_bounds__(kThreads) direction_kernel(int64_t N, const uint8_t* __restrict__ known,
+                                                             const T* __restrict__ y, T* __restrict__ p,
+                                                             const Scal* sc, CoarseDev C, int mode) {
+  if (mode == 0 && sc->done) return;
+  constexpr int nr = Modes<D>::nr;
+  const T beta = (T)sc->beta;
+  const T* ec = sizeof(T) == 4 ? (const T*)C.ecf : (const T*)C.ec;
+  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < N; i += (int64_t)gridDim.x * blockDim.x) {
+    const int64_t a = i / D;
+    T z = y[i];
+    if (!known[i]) z += mode_row<D, T>((int)(i - a * D), C.off[a], ec + (int64_t)C.agg[a] * nr);
+    p[i] = z + beta * p[i];
   }
 }
 
@@ -1329,7 +1417,7 @@ SysT<float> sys_t<float>(const gfea_system* s) {
 int launch_resid(const gfea_system* s, int G, const double* b, const double* x, PcgWork& w, bool kn,
                  cudaStream_t st) {
   const SysT<double> S = sys_t<double>(s);
-  const int grid = grid_nodes(s->n_nodes, G);
+  const int grid = grid_nodes(s->n_nodes, G <= 4 ? 4 : 8);
   const int64_t N = s->n_nodes * s->dof_n;
   const float* v32 = s->vals32;
   float* x32 = nullptr;
@@ -1338,9 +1426,20 @@ int launch_resid(const gfea_system* s, int G, const double* b, const double* x, 
     cast_kernel<float><<<grid_elems(N), kThreads, 0, st>>>(x, x32, N);
     GFEA_LAUNCH_CHECK();
   }
-#define GFEA_RESID(KN_, AB_)                                                                                   \
-  GFEA_DG_SWITCH(s->dof_n, G, (resid_kernel<DD, GG, double, KN_, AB_><<<grid, kThreads, 0, st>>>(               \
-                                  S, v32, x32, b, x, w.r64, w.partials, w.sc)))
+  // scalar systems: a lane group per row (a component per lane would leave
+  // every lane with a row of its own)
+#define GFEA_RESID(KN_, AB_)                                                                                     \
+  switch (s->dof_n) {                                                                                            \
+    case 2: resid_comp_kernel<2, KN_, AB_><<<kSMs * 3, kThreads, 0, st>>>(S, v32, x32, b, x, w.r64, w.partials, w.sc); break; \
+    case 3: resid_comp_kernel<3, KN_, AB_><<<kSMs * 3, kThreads, 0, st>>>(S, v32, x32, b, x, w.r64, w.partials, w.sc); break; \
+    case 1:                                                                                                      \
+      if (G <= 4)                                                                                                \
+        resid_kernel<1, 4, double, KN_, AB_><<<grid, kThreads, 0, st>>>(S, v32, x32, b, x, w.r64, w.partials, w.sc); \
+      else                                                                                                       \
+        resid_kernel<1, 8, double, KN_, AB_><<<grid, kThreads, 0, st>>>(S, v32, x32, b, x, w.r64, w.partials, w.sc); \
+      break;                                                                                                     \
+    default: return GFEA_ERR_ARG;                                                                                \
+  }
   if (kn) {
     if (x32) { GFEA_RESID(true, true); } else { GFEA_RESID(true, false); }
   } else {
@@ -1493,8 +1592,15 @@ int launch_apply(const gfea_system* s, int G, PcgWork& w, const T* p, cudaStream
   return GFEA_OK;
 }
 
+// The iteration's product.  Block-Jacobi: p_new = z + beta p_old first; with
+// the coarse level p_old already holds the direction.
 template <typename T>
 int launch_dir(const gfea_system* s, int G, PcgWork& w, const T* p_old, T* p_new, cudaStream_t st) {
+  if (w.coarse) {
+    const int e = launch_apply<T>(s, G, w, p_old, st);
+    if (e) return e;
+    return prof_mark(st, kTagApply);
+  }
   if (!w.packed) {  // one kernel: the direction formed inside the SpMV
     const int e = launch_apply<T>(s, G, w, p_old, st, (const T*)w.z, p_new);
     if (e) return e;
@@ -1510,16 +1616,16 @@ int launch_dir(const gfea_system* s, int G, PcgWork& w, const T* p_old, T* p_new
   return prof_mark(st, kTagApply);
 }
 
-// z = M^-1 r (with the x, r update in mode 0): update_kernel alone, or the
-// restriction / coarse solve / prolongation sequence of the two-level
-// preconditioner.
+// Block-Jacobi: z = D^-1 r (with the x, r update in mode 0).  Two-level: x, r,
+// y = D^-1 r and the restriction; the coarse solve and beta; the direction.
 template <typename T>
 int launch_precond(const gfea_system* s, PcgWork& w, T* x, T* p, int mode, cudaStream_t st) {
   if (!w.coarse) return launch_update<T>(s, w, x, p, mode, st);
   const int grid = grid_elems(s->n_nodes);
-  GFEA_D_SWITCH(s->dof_n, (update_r_kernel<DD, T><<<grid, kThreads, 0, st>>>(s->n_nodes, s->known, x,
-                                                                              (T*)w.r, p, (const T*)w.Ap, w.sc, w.C,
-                                                                              mode)));
+  const int64_t N = s->n_nodes * s->dof_n;
+  GFEA_D_SWITCH(s->dof_n, (update_r_kernel<DD, T><<<grid, kThreads, 0, st>>>(
+                              s->n_nodes, s->known, (const T*)w.dinv, x, (T*)w.r, (T*)w.z, p, (const T*)w.Ap,
+                              w.partials + 2 * kMaxBlocks, w.sc, w.C, mode)));
   GFEA_LAUNCH_CHECK();
   int e = prof_mark(st, kTagRestrict);
   if (e) return e;
@@ -1527,16 +1633,14 @@ int launch_precond(const gfea_system* s, PcgWork& w, T* x, T* p, int mode, cudaS
     rc_sum_kernel<<<(int)ceil_div(w.C.nc, kThreads), kThreads, 0, st>>>(w.C, w.sc, mode);
     GFEA_LAUNCH_CHECK();
   }
-  coarse_gemv_kernel<<<std::min(w.C.nc, 8 * kSMs), kGemvThreads, 0, st>>>(w.C, w.sc, mode);
+  coarse_gemv_kernel<<<std::min(w.C.nc, 8 * kSMs), kGemvThreads, 0, st>>>(w.C, w.partials, w.sc, mode);
   GFEA_LAUNCH_CHECK();
   e = prof_mark(st, kTagGemv);
   if (e) return e;
-  GFEA_D_SWITCH(s->dof_n, (finish_z_kernel<DD, T><<<grid, kThreads, 0, st>>>(s->n_nodes, s->known,
-                                                                              (const T*)w.dinv, (const T*)w.r,
-                                                                              (T*)w.z, w.partials + 2 * kMaxBlocks,
-                                                                              w.sc, w.C, mode)));
+  GFEA_D_SWITCH(s->dof_n, (direction_kernel<DD, T><<<grid_elems(N), kThreads, 0, st>>>(N, s->known, (const T*)w.z, p,
+                                                                                       w.sc, w.C, mode)));
   GFEA_LAUNCH_CHECK();
-  return prof_mark(st, kTagFinish);
+  return prof_mark(st, kTagDir);
 }
 
 // Coarse level of the two-level preconditioner: aggregates = cells of a grid
@@ -1797,12 +1901,11 @@ int capture_iterations(const gfea_system* s, int G, PcgWork& w, T* x, T* p0, T* 
   }
   cudaGraph_t g = nullptr;
   const cudaError_t ce = cudaStreamEndCapture(cs, &g);
-  // kernels per iteration: direction + SpMV (one kernel without packed
-  // tiles), then update (block-Jacobi) or
-  // update/restrict + restriction sum (with restriction copies) + coarse
-  // GEMV + finish (two-level); counted when the graph runs, not when it is
-  // captured
-  w.gkernels = (long long)kGraphIters * ((w.packed ? 2 : 1) + (w.coarse ? (w.C.ncopies > 1 ? 4 : 3) : 1));
+  // kernels per iteration, counted when the graph runs, not when it is
+  // captured: SpMV, update/restrict, restriction sum (with restriction
+  // copies), coarse GEMV and direction (two-level); direction, SpMV (one
+  // kernel without packed tiles) and update (block-Jacobi)
+  w.gkernels = (long long)kGraphIters * (w.coarse ? (w.C.ncopies > 1 ? 5 : 4) : (w.packed ? 3 : 2));
   launch_counter().fetch_sub(w.gkernels);
   if (e || ce != cudaSuccess || !g) {
     if (g) cudaGraphDestroy(g);
@@ -1835,6 +1938,8 @@ int pcg_loop(const gfea_system* s, int G, PcgWork& w, T* x, int check, bool grow
   // iteration j reads direction buf[j % 2] and writes buf[(j + 1) % 2]; launches
   // after the device set 'done' are no-ops, so the current direction follows
   // from the number of iterations actually performed
+  // (the two-level iteration updates one buffer in place)
+  if (w.coarse) pb = pa;
   T* buf[2] = {pa, pb};
   KernelProfile& P = prof();
   ChunkEvents& E = chunk_events();
@@ -1988,7 +2093,11 @@ int refine_solve(const gfea_system* s, const double* b, double* x, const gfea_pc
   // host checks: every check_every iterations, or (check_every <= 0) after a
   // first chunk sized from the previous reliable-update cycle, then doubling
   const bool adaptive = o->check_every <= 0;
-  int check = adaptive ? 16 : o->check_every;
+  // staged operators: an iteration takes ~0.1 ms and more, a check ~15 us, and
+  // the launches after convergence ~8 us an iteration, so short chunks cost
+  // least (516 iterations were launched for 222 when chunks grew)
+  const bool grow = adaptive && !w.packed;
+  int check = grow ? 16 : (adaptive ? 2 * kGraphIters : o->check_every);
   const bool fp64 = sizeof(T) == 8;
   const double eps64 = 2.220446049250313e-16;
   // reliable update after the iterated residual fell by delta: inner_rtol
@@ -2105,8 +2214,8 @@ int refine_solve(const gfea_system* s, const double* b, double* x, const gfea_pc
   int stall = 0;
   int iters0 = 0;
   for (int upd = 0;; ++upd) {
-    e = pcg_loop<T>(s, G, w, (T*)w.dx, check, adaptive, &hs, pa, pb, iters0, rr, st);
-    if (adaptive) {
+    e = pcg_loop<T>(s, G, w, (T*)w.dx, check, grow, &hs, pa, pb, iters0, rr, st);
+    if (grow) {
       const int cycle = hs.iters - iters0;
       check = cycle + 2 < 4 ? 4 : (cycle + 2 > 64 ? 64 : cycle + 2);
     }
