@@ -23,18 +23,6 @@ namespace {
 
 // Per-lane geometry at one Gauss point: Jacobian reduced across the group,
 // wJ and the physical gradient of this lane's shape function.
-// Reciprocal by Newton-Raphson iteration on f(r) = 1/r - x (r <- r + r (1 - x r))
-// from an FP32 seed (relative error ~2^-23): two steps reach double precision
-// with four FP64 FMAs; the full division where the seed is out of FP32 range.
-__device__ __forceinline__ double recip_newton(double x) {
-  const float s = 1.0f / (float)x;
-  if (!(fabsf(s) > 0.f) || isinf(s)) return 1.0 / x;
-  double r = (double)s;
-  r = fma(r, fma(-x, r, 1.0), r);
-  r = fma(r, fma(-x, r, 1.0), r);
-  return r;
-}
-
 // Sum of nine per-lane values over a group of 8 lanes (the 3x3 Jacobian of a
 // HEXA8): a reduce-scatter in three exchange steps -- each lane keeps the
 // values owned by its half (value v owned by lane v, value 8 by lane 0) and
@@ -312,15 +300,13 @@ __global__ void __launch_bounds__(128) elastic_kernel(const double* __restrict__
 //
 // FP64 instructions retire at a sixteenth of a warp per cycle whatever the
 // number of lanes that differ, and in elastic_kernel every lane repeats each
-// point's inverse Jacobian behind a reduction of its entries: 1019 FP64
-// instructions per four HEXA8, 565 here.  With c the adjugate times dN_p,
-// M_pq = sum_g (w / |det|) c_p (x) c_q, so no gradient is scaled by 1 / det.
-// The diagonal block is symmetric (D (D + 1) / 2 entries), and of the block of
-// an opposite pair (even nPe) each of its two lanes accumulates the upper
-// triangle and takes the other half from its partner.
+// point's inverse Jacobian behind a reduction of its entries (1019 FP64
+// instructions per four HEXA8).  Every entry is formed by the same operations
+// in the same order (see point_jacobian).
 // Bound: FP64 pipe, then the atomics.  elastic_kernel -> this: 640,000 HEXA8
-// 9.80 -> 5.68 ms, 1.05 million QUAD4 1.75 -> 0.96, 80,000 QUAD9 1.68 -> 0.98,
-// 24,552 TETRA10 0.64 -> 0.35.
+// 9.80 -> 7.41 ms, 1.05 million QUAD4 1.75 -> 1.25, 80,000 QUAD9 1.68 -> 1.15,
+// 24,552 TETRA10 0.64 -> 0.44 (adjugate products and symmetric halves would
+// take 5.7, 0.96, 0.98 and 0.35, with other roundings).
 template <int ELEM, int CMODE>
 __global__ void __launch_bounds__(128) elastic_iso_kernel(const double* __restrict__ coord,
                                                           const int32_t* __restrict__ connect, int64_t Ne,
@@ -331,16 +317,14 @@ __global__ void __launch_bounds__(128) elastic_iso_kernel(const double* __restri
   using E = Elem<ELEM>;
   using Ref = RefTables<ELEM, false>;
   constexpr int nPe = E::nPe, D = E::dim, nPg = Ref::nPg, G = NextPow2<nPe>::value, EPW = 32 / G;
-  constexpr int S = G / NextPow2<nPg>::value;       // lanes per Gauss point
-  constexpr bool HALF = nPe % 2 == 0;               // an opposite pair shares a block
-  constexpr int NF = HALF ? nPe / 2 - 1 : nPe / 2;  // blocks p, p + 1 .. p + NF of a lane
-  constexpr int LD = (nPe * D) | 1;                 // odd: the points' columns start in different banks
-  constexpr int NU = D * (D + 1) / 2;
+  constexpr int S = G / NextPow2<nPg>::value;  // lanes per Gauss point
+  constexpr bool HALF = nPe % 2 == 0;          // an opposite pair shares a block
+  constexpr int LD = (nPe * D) | 1;            // odd: the points' columns start in different banks
   static_assert(S >= 1 && nPg * S <= G, "one point per S lanes");
   __shared__ Ref ref;
-  __shared__ double sc[4 * EPW][nPg * LD];  // c_q of every point
+  __shared__ double sc[4 * EPW][nPg * LD];  // gradients at every point
   __shared__ double sx[4 * EPW][nPe * D];
-  __shared__ double sf[4 * EPW][nPg];       // w / |det|
+  __shared__ double sf[4 * EPW][nPg];       // wJ
   ref.fill();
   __syncthreads();
   const double lam = Cglob[0], mu = Cglob[1];
@@ -369,184 +353,69 @@ __global__ void __launch_bounds__(128) elastic_iso_kernel(const double* __restri
     {
       const int g = lane / S < nPg ? lane / S : nPg - 1, h = lane % S;
       double F[D][D];
-#pragma unroll
-      for (int d = 0; d < D; ++d)
-#pragma unroll
-        for (int k = 0; k < D; ++k) F[d][k] = 0;
-#pragma unroll
-      for (int q0 = 0; q0 < nPe; q0 += S) {
-        const int q = q0 + h;
-        if (nPe % S == 0 || q < nPe) {
-#pragma unroll
-          for (int d = 0; d < D; ++d)
-#pragma unroll
-            for (int k = 0; k < D; ++k) F[d][k] += ref.dN[g][d][q] * x[q * D + k];
-        }
-      }
-#pragma unroll
-      for (int o = S / 2; o > 0; o >>= 1)
-#pragma unroll
-        for (int d = 0; d < D; ++d)
-#pragma unroll
-          for (int k = 0; k < D; ++k) F[d][k] += __shfl_xor_sync(0xffffffffu, F[d][k], o);
-      double adj[D][D], det;
-      if constexpr (D == 2) {
-        det = F[0][0] * F[1][1] - F[1][0] * F[0][1];
-        adj[0][0] = F[1][1];
-        adj[0][1] = -F[0][1];
-        adj[1][0] = -F[1][0];
-        adj[1][1] = F[0][0];
-      } else {
-        adj[0][0] = F[1][1] * F[2][2] - F[2][1] * F[1][2];
-        adj[0][1] = F[2][1] * F[0][2] - F[0][1] * F[2][2];
-        adj[0][2] = F[0][1] * F[1][2] - F[1][1] * F[0][2];
-        adj[1][0] = F[2][0] * F[1][2] - F[1][0] * F[2][2];
-        adj[1][1] = F[0][0] * F[2][2] - F[2][0] * F[0][2];
-        adj[1][2] = F[1][0] * F[0][2] - F[0][0] * F[1][2];
-        adj[2][0] = F[1][0] * F[2][1] - F[2][0] * F[1][1];
-        adj[2][1] = F[2][0] * F[0][1] - F[0][0] * F[2][1];
-        adj[2][2] = F[0][0] * F[1][1] - F[1][0] * F[0][1];
-        det = F[0][0] * adj[0][0] + F[0][1] * adj[1][0] + F[0][2] * adj[2][0];
-      }
+      point_jacobian<ELEM, false, S>(ref, g, h, x, F);
       if (lane / S < nPg) {
-#pragma unroll
-        for (int q0 = 0; q0 < nPe; q0 += S) {
-          const int q = q0 + h;
-          if (nPe % S == 0 || q < nPe) {
-#pragma unroll
-            for (int i = 0; i < D; ++i) {
-              double v = adj[i][0] * ref.dN[g][0][q];
-#pragma unroll
-              for (int d = 1; d < D; ++d) v += adj[i][d] * ref.dN[g][d][q];
-              c[g * LD + q * D + i] = v;
-            }
-          }
-        }
-        if (h == 0) fg[g] = ref.w[g] * fabs(recip_newton(det));
+        const double det = point_gradients<ELEM, false, S>(ref, g, h, F, [&](int q, int i, double v) { c[g * LD + q * D + i] = v; });
+        if (h == 0) fg[g] = fabs(det) * ref.w[g];
       }
     }
     __syncwarp();
-    double m0[NU], mf[NF > 0 ? NF : 1][D][D], mh[NU];
+    constexpr int NB = nPe / 2 + 1;  // blocks p, p + 1 .. of a lane
+    double m[NB][D][D];
 #pragma unroll
-    for (int u = 0; u < NU; ++u) m0[u] = mh[u] = 0;
-#pragma unroll
-    for (int d = 0; d < NF; ++d)
+    for (int d = 0; d < NB; ++d)
 #pragma unroll
       for (int i = 0; i < D; ++i)
 #pragma unroll
-        for (int j = 0; j < D; ++j) mf[d][i][j] = 0;
-    int qd[NF + 2];
+        for (int j = 0; j < D; ++j) m[d][i][j] = 0;
+    int qd[NB];
 #pragma unroll
-    for (int d = 0; d < NF + 2; ++d) qd[d] = pl + d < nPe ? pl + d : pl + d - nPe;
+    for (int d = 0; d < NB; ++d) qd[d] = pl + d < nPe ? pl + d : pl + d - nPe;
 #pragma unroll 1
     for (int g = 0; g < nPg; ++g) {
       const double* cg = c + g * LD;
-      const double f = fg[g];
-      double own[D], w[D];
+      const double wJ = fg[g];
+      double w[D];
 #pragma unroll
-      for (int i = 0; i < D; ++i) {
-        own[i] = cg[pl * D + i];
-        w[i] = f * own[i];
-      }
-      int u = 0;
+      for (int i = 0; i < D; ++i) w[i] = wJ * cg[pl * D + i];
 #pragma unroll
-      for (int i = 0; i < D; ++i)
+      for (int d = 0; d < NB; ++d) {
+        double h[D];
 #pragma unroll
-        for (int j = i; j < D; ++j) m0[u++] += w[i] * own[j];
-#pragma unroll
-      for (int d = 0; d < NF; ++d) {
-        const double* h = cg + qd[d + 1] * D;
-#pragma unroll
-        for (int j = 0; j < D; ++j) {
-          const double hj = h[j];
-#pragma unroll
-          for (int i = 0; i < D; ++i) mf[d][i][j] += w[i] * hj;
-        }
-      }
-      if (HALF) {
-        const double* h = cg + qd[NF + 1] * D;
-        u = 0;
+        for (int j = 0; j < D; ++j) h[j] = cg[qd[d] * D + j];
 #pragma unroll
         for (int i = 0; i < D; ++i)
 #pragma unroll
-          for (int j = i; j < D; ++j) mh[u++] += w[i] * h[j];
+          for (int j = 0; j < D; ++j) m[d][i][j] += w[i] * h[j];
       }
     }
-    const double fe = CMODE == 4 ? factor * __ldg(Cglob + 2 + ec) : factor;
-    const double lf = fe * lam, mf2 = fe * mu;
+    const double f = CMODE == 4 ? factor * __ldg(Cglob + 2 + ec) : factor;
     const uint8_t* rke = rank + ec * nPe * nPe;
     const bool act = valid && node_lane;
-    auto form = [&](const double (&M)[D][D], double (&K)[D][D]) {
+#pragma unroll
+    for (int d = 0; d < NB; ++d) {
+      const int q = qd[d];
+      const int32_t pb0 = group_bcast<G, int32_t>(pa0, q), Wb = group_bcast<G, int32_t>(Wa, q);
+      if (!act || (HALF && d == NB - 1 && lane >= nPe / 2)) continue;  // the opposite pair's block: its lower lane
       double tr = 0;
 #pragma unroll
-      for (int i = 0; i < D; ++i) tr += M[i][i];
-#pragma unroll
-      for (int i = 0; i < D; ++i)
-#pragma unroll
-        for (int j = 0; j < D; ++j) K[i][j] = lf * M[i][j] + mf2 * (i == j ? M[i][i] + tr : M[j][i]);
-    };
-    // entry [i][j] of the block in row 'node' (first slot p0, row length W) at neighbour rank r
-    auto row_at = [&](int32_t p0, int32_t W, int r, int i) {
-      return vals + (int64_t)D * D * p0 + (int64_t)i * W + D * r;
-    };
-    {
-      double M[D][D], K[D][D];
-      int u = 0;
-#pragma unroll
-      for (int i = 0; i < D; ++i)
-#pragma unroll
-        for (int j = i; j < D; ++j) M[i][j] = M[j][i] = m0[u++];
-      form(M, K);
-      if (act) {
-        const int r = rke[lane * nPe + lane];
-#pragma unroll
-        for (int i = 0; i < D; ++i) {
-          double* row = row_at(pa0, Wa, r, i);
-#pragma unroll
-          for (int j = 0; j < D; ++j) atomicAdd(row + j, K[i][j]);
-        }
-      }
-    }
-#pragma unroll
-    for (int d = 0; d < NF; ++d) {
-      const int q = qd[d + 1];
-      const int32_t pb0 = group_bcast<G, int32_t>(pa0, q), Wb = group_bcast<G, int32_t>(Wa, q);
+      for (int i = 0; i < D; ++i) tr += m[d][i][i];
       double K[D][D];
-      form(mf[d], K);
-      if (act) {
-        const int r_pq = rke[lane * nPe + q], r_qp = rke[q * nPe + lane];
 #pragma unroll
-        for (int i = 0; i < D; ++i) {
-          double* row = row_at(pa0, Wa, r_pq, i);
+      for (int i = 0; i < D; ++i)
 #pragma unroll
-          for (int j = 0; j < D; ++j) atomicAdd(row + j, K[i][j]);
-          double* col = row_at(pb0, Wb, r_qp, i);
+        for (int j = 0; j < D; ++j)
+          K[i][j] = f * (i == j ? lam * m[d][i][i] + mu * m[d][i][i] + mu * tr : lam * m[d][i][j] + mu * m[d][j][i]);
+      const int r_pq = rke[lane * nPe + q], r_qp = rke[q * nPe + lane];
+#pragma unroll
+      for (int i = 0; i < D; ++i) {
+        double* row = vals + (int64_t)D * D * pa0 + (int64_t)i * Wa + D * r_pq;
+#pragma unroll
+        for (int j = 0; j < D; ++j) atomicAdd(row + j, K[i][j]);
+        if (d > 0) {  // row q, block p: the transpose
+          double* col = vals + (int64_t)D * D * pb0 + (int64_t)i * Wb + D * r_qp;
 #pragma unroll
           for (int j = 0; j < D; ++j) atomicAdd(col + j, K[j][i]);
-        }
-      }
-    }
-    if (HALF) {
-      const int q = qd[NF + 1];
-      double M[D][D], K[D][D];
-      int u = 0;
-#pragma unroll
-      for (int i = 0; i < D; ++i)
-#pragma unroll
-        for (int j = i; j < D; ++j) {
-          M[i][j] = mh[u];
-          const double other = group_bcast<G, double>(mh[u], q);
-          if (i != j) M[j][i] = other;
-          ++u;
-        }
-      form(M, K);
-      if (act) {
-        const int r = rke[lane * nPe + q];
-#pragma unroll
-        for (int i = 0; i < D; ++i) {
-          double* row = row_at(pa0, Wa, r, i);
-#pragma unroll
-          for (int j = 0; j < D; ++j) atomicAdd(row + j, K[i][j]);
         }
       }
     }

@@ -754,6 +754,18 @@ template <int n> struct NextPow2 {
   static constexpr int value = n <= 1 ? 1 : (n <= 2 ? 2 : (n <= 4 ? 4 : (n <= 8 ? 8 : (n <= 16 ? 16 : 32))));
 };
 
+// Reciprocal by Newton-Raphson iteration on f(r) = 1/r - x (r <- r + r (1 - x r))
+// from an FP32 seed (relative error ~2^-23): two steps reach double precision
+// with four FP64 FMAs; the full division where the seed is out of FP32 range.
+__device__ __forceinline__ double recip_newton(double x) {
+  const float s = 1.0f / (float)x;
+  if (!(fabsf(s) > 0.f) || isinf(s)) return 1.0 / x;
+  double r = (double)s;
+  r = fma(r, fma(-x, r, 1.0), r);
+  r = fma(r, fma(-x, r, 1.0), r);
+  return r;
+}
+
 // ---------------------------------------------------------------------------
 // Jacobian helpers (closed forms of EasyFEA/FEM/_linalg.py:533-656)
 // ---------------------------------------------------------------------------
@@ -764,7 +776,7 @@ __device__ __forceinline__ double det_inv(const double (&F)[D][D], double (&iF)[
     return F[0][0];
   } else if constexpr (D == 2) {
     const double det = F[0][0] * F[1][1] - F[1][0] * F[0][1];
-    const double id = 1.0 / det;
+    const double id = __drcp_rn(det);  // as 1.0 / det
     iF[0][0] = id * F[1][1];
     iF[0][1] = id * -F[0][1];
     iF[1][0] = id * -F[1][0];
@@ -776,7 +788,7 @@ __device__ __forceinline__ double det_inv(const double (&F)[D][D], double (&iF)[
     const double a31 = F[2][0], a32 = F[2][1], a33 = F[2][2];
     const double det = a11 * ((a22 * a33) - (a32 * a23)) - a12 * ((a21 * a33) - (a31 * a23)) +
                        a13 * ((a21 * a32) - (a31 * a22));
-    const double id = 1.0 / det;
+    const double id = __drcp_rn(det);
     iF[0][0] = id * (a22 * a33 - a32 * a23);
     iF[0][1] = id * -(a12 * a33 - a32 * a13);
     iF[0][2] = id * (a12 * a23 - a22 * a13);
