@@ -10,6 +10,14 @@
 // launch).  Iterations are FP32 (values, vectors, block-Jacobi) with FP64 dot
 // products, scalars and reliable-update residuals, or FP64 throughout.
 //
+// The phases of an iteration are bound by chains of L2 round trips (8 or 16
+// warps per SM), so each batches the loads of several rows, nodes or
+// neighbour passes before it uses the first.  32 random-material cantilevers
+// of 2000 to 50000 unknowns, mixed precision, assembly included: 26.8 ms with
+// one neighbour pass and one node at a time and 256 threads throughout, 23.9
+// with the batched loads, 16.8 with the wide clusters; 64 of 3000 unknowns
+// 9.2 -> 6.9 ms.
+//
 // Cross-CTA reads of vectors written inside the launch use L2-only loads
 // (ld.global.cg), so no stale L1 line is ever consulted; the cluster barrier
 // orders the writes (release/acquire at cluster scope).
@@ -30,7 +38,19 @@ namespace gfea {
 namespace {
 
 constexpr int kCL = 8;    // CTAs per cluster (portable cluster size)
-constexpr int kBT = 256;  // threads per CTA
+
+// Threads per CTA: 256 (two CTAs per SM), or 512 (one) for the systems of at
+// least kWideValues stored values.  A cluster's passes over its rows are bound
+// by L2 latency at either width, so twice the warps shorten a solve (24021
+// QUAD4 nodes: 19.0 -> 14.4 ms, 5425: 5.4 -> 4.8 ms) for twice the SMs: worth
+// it where a large system is the tail of the launch, not for many small ones
+// (64 systems of 3000 unknowns: 6.9 ms narrow, 13.3 ms wide; 40 of 20000:
+// 24.9 and 27.0).  The width follows the system's own size alone, so its
+// result does not depend on the others in the launch.
+constexpr int kNarrow = 256, kWide = 512;
+constexpr int64_t kWideValues = 400000;
+
+__host__ __device__ inline int64_t stored_values(const gfea_batch_instance& I) { return I.n_pairs * I.dof_n * I.dof_n; }
 
 size_t a256(size_t b) { return (b + 255) & ~size_t(255); }
 
@@ -71,22 +91,38 @@ struct Ctx {
   cg::cluster_group cl;
   unsigned rank;
   double* slots;  // this CTA's 2 x 4 reduction slots
-  double* sh;     // block_sum scratch
+  double* sh;     // warp partials, 4 values
   int phase;
 };
 
 // Cluster-wide sum of NV values; every thread of every CTA gets the same result.
+// (c.sh is free again once the cluster barrier has been passed.)
 template <int NV>
 __device__ void csum(Ctx& c, const double (&v)[NV], double (&out)[NV]) {
+  const int warps = blockDim.x >> 5;
   double* slot = c.slots + (c.phase & 1) * 4;
+  const int wp = threadIdx.x >> 5, l = threadIdx.x & 31;
 #pragma unroll
   for (int k = 0; k < NV; ++k) {
-    const double s = block_sum(v[k], c.sh);
-    if (threadIdx.x == 0) slot[k] = s;
+    double t = v[k];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+    if (l == 0) c.sh[k * (kWide / 32) + wp] = t;
+  }
+  __syncthreads();
+  if (wp == 0) {
+#pragma unroll
+    for (int k = 0; k < NV; ++k) {
+      double t = l < warps ? c.sh[k * (kWide / 32) + l] : 0.0;
+#pragma unroll
+      for (int o = kWide / 64; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+      if (l == 0) slot[k] = t;
+    }
   }
   c.cl.sync();
 #pragma unroll
   for (int k = 0; k < NV; ++k) out[k] = 0;
+#pragma unroll
   for (unsigned r = 0; r < (unsigned)kCL; ++r) {
     const double* rs = c.cl.map_shared_rank(slot, r);
 #pragma unroll
@@ -97,32 +133,95 @@ __device__ void csum(Ctx& c, const double (&v)[NV], double (&out)[NV]) {
 
 // FP64 residual r64 = P(b - A64 x) over the cluster; partials r.r, ||P(b - A x_c)||^2,
 // ||P(|A||x| + |b|)||^2 accumulated into v[0..2].
+//
+// The three products share one pass over the row, two rows at a time with the
+// loads of kPasses neighbour passes in flight (bound by the chain of L2 round
+// trips, as node_rows_multi below).
+constexpr int kPasses = 3;
+
 template <int D, int G>
-__device__ void resid64(const SysT<double>& S, const double* b, const double* x, double* r64, int64_t grp,
+__device__ __noinline__ void resid64(const SysT<double>& S, const double* b, const double* x, double* r64, int64_t grp,
                         int64_t ngrp, int lane, double (&v)[4]) {
+  constexpr int LA = G - G % D;
+  constexpr int NPP = LA / D;
+  constexpr int R = D < 3 ? 2 : 1;
   const int64_t Nn = S.Nn;
   const int64_t sub = grp % (32 / G);
-  for (int64_t a0 = grp - sub; a0 < Nn; a0 += ngrp) {
-    const int64_t a = a0 + sub;
-    const int64_t ac = a < Nn ? a : Nn - 1;
-    double all[D], kn[D], ab[D];
-    node_rows<D, G, double, double>(ac, lane, S, [&](int64_t cc) { return ldcg(x + cc); }, all);
-    node_rows<D, G, double, double>(ac, lane, S,
-                                    [&](int64_t cc) { return S.known[cc] ? ldcg(x + cc) : 0.0; }, kn);
-    node_rows<D, G, double, double, true>(ac, lane, S, [&](int64_t cc) { return fabs(ldcg(x + cc)); }, ab);
-    if (a < Nn && lane == 0) {
+  const int j = lane % D;
+  for (int64_t a0 = grp - sub; a0 < Nn; a0 += R * ngrp) {
+    int64_t an[R];
+    int32_t p0[R], nb[R];
+    double all[R][D], kn[R][D], ab[R][D];
+    int32_t maxnb = 0;
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      an[r] = a0 + sub + r * ngrp;
+      const int64_t ac = an[r] < Nn ? an[r] : Nn - 1;
+      p0[r] = S.node_ptr[ac];
+      nb[r] = S.node_ptr[ac + 1] - p0[r];
+      maxnb = nb[r] > maxnb ? nb[r] : maxnb;
+#pragma unroll
+      for (int i = 0; i < D; ++i) all[r][i] = kn[r][i] = ab[r][i] = 0;
+    }
+    if (lane < LA) {
+      for (int32_t k0 = lane / D, t0 = lane; k0 < maxnb; k0 += kPasses * NPP, t0 += kPasses * LA) {
+        int32_t c[kPasses][R];
+        double val[kPasses][R][D], xv[kPasses][R];
+        bool known[kPasses][R];
+#pragma unroll
+        for (int u = 0; u < kPasses; ++u)
+#pragma unroll
+          for (int r = 0; r < R; ++r) {
+            const int32_t k = k0 + u * NPP;
+            const bool in = k < nb[r];
+            c[u][r] = in ? __ldg(S.nbr + p0[r] + k) : -1;
+#pragma unroll
+            for (int i = 0; i < D; ++i)
+              val[u][r][i] =
+                  in ? __ldg(S.vals + (int64_t)D * D * p0[r] + (int64_t)i * D * nb[r] + t0 + u * LA) : 0.0;
+          }
+#pragma unroll
+        for (int u = 0; u < kPasses; ++u)
+#pragma unroll
+          for (int r = 0; r < R; ++r) {
+            const int64_t col = (int64_t)c[u][r] * D + j;
+            xv[u][r] = c[u][r] >= 0 ? ldcg(x + col) : 0.0;
+            known[u][r] = c[u][r] >= 0 ? S.known[col] : false;
+          }
+#pragma unroll
+        for (int u = 0; u < kPasses; ++u)
+#pragma unroll
+          for (int r = 0; r < R; ++r)
+#pragma unroll
+            for (int i = 0; i < D; ++i) {
+              all[r][i] += val[u][r][i] * xv[u][r];
+              kn[r][i] += val[u][r][i] * (known[u][r] ? xv[u][r] : 0.0);
+              ab[r][i] += fabs(val[u][r][i]) * fabs(xv[u][r]);
+            }
+      }
+    }
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
 #pragma unroll
       for (int i = 0; i < D; ++i) {
-        const int64_t dof = a * D + i;
-        const bool unk = !S.known[dof];
-        const double bi = __ldg(b + dof);
-        const double ri = unk ? bi - all[i] : 0.0;
-        const double rci = unk ? bi - kn[i] : 0.0;
-        const double ai = unk ? ab[i] + fabs(bi) : 0.0;
-        r64[dof] = ri;
-        v[0] += ri * ri;
-        v[1] += rci * rci;
-        v[2] += ai * ai;
+        all[r][i] = group_sum<G, double>(all[r][i]);
+        kn[r][i] = group_sum<G, double>(kn[r][i]);
+        ab[r][i] = group_sum<G, double>(ab[r][i]);
+      }
+      if (an[r] < Nn && lane == 0) {
+#pragma unroll
+        for (int i = 0; i < D; ++i) {
+          const int64_t dof = an[r] * D + i;
+          const bool unk = !S.known[dof];
+          const double bi = __ldg(b + dof);
+          const double ri = unk ? bi - all[r][i] : 0.0;
+          const double rci = unk ? bi - kn[r][i] : 0.0;
+          const double ai = unk ? ab[r][i] + fabs(bi) : 0.0;
+          r64[dof] = ri;
+          v[0] += ri * ri;
+          v[1] += rci * rci;
+          v[2] += ai * ai;
+        }
       }
     }
   }
@@ -154,53 +253,56 @@ __device__ void restart_rz(const gfea_batch_instance& I, const BatchBuf<T>& w, i
 }
 
 // node_rows for R nodes at once (one G-lane group): the index, value and
-// gathered-vector loads of the R rows in a pass are independent and issued
-// together.  A cluster runs 16 warps per SM, too few to hide the three
-// dependent L2 round trips of a row (row pointer, neighbour index, gather)
-// one row at a time.
+// gathered-vector loads of the R rows in kPasses neighbour passes are
+// independent and issued together.  A cluster runs 16 warps per SM, too few to
+// hide the three dependent L2 round trips of a row (row pointer, neighbour
+// index, gather) one row at a time; a QUAD4 or HEXA8 interior row has three
+// passes, so it takes the three round trips once.  self: xf at the lane's own
+// component of each row.
 template <int D, int G, typename T, bool DIFF, int R, typename XF>
-__device__ __forceinline__ void node_rows_multi(const int64_t (&a)[R], int lane, const SysT<T>& S, XF xf,
-                                                T (&acc)[R][D]) {
+__device__ __forceinline__ void node_rows_multi(const int64_t (&a)[R], const int32_t (&p0)[R], const int32_t (&nb)[R],
+                                                int lane, const SysT<T>& S, XF xf, T (&acc)[R][D], T (&self)[R]) {
   constexpr int LA = G - G % D;
   constexpr int NPP = LA / D;
   const int j = lane % D;
-  int32_t p0[R], nb[R];
-#pragma unroll
-  for (int r = 0; r < R; ++r) {
-    p0[r] = S.node_ptr[a[r]];
-    nb[r] = S.node_ptr[a[r] + 1] - p0[r];
-  }
 #pragma unroll
   for (int r = 0; r < R; ++r)
 #pragma unroll
     for (int i = 0; i < D; ++i) acc[r][i] = 0;
   if (lane < LA) {
-    T self[R];
 #pragma unroll
-    for (int r = 0; r < R; ++r) self[r] = DIFF ? xf(a[r] * D + j) : (T)0;
+    for (int r = 0; r < R; ++r) self[r] = xf(a[r] * D + j);
     int32_t maxnb = nb[0];
 #pragma unroll
     for (int r = 1; r < R; ++r) maxnb = nb[r] > maxnb ? nb[r] : maxnb;
-    for (int32_t k = lane / D, t = lane; k < maxnb; k += NPP, t += LA) {
-      int32_t c[R];
+    for (int32_t k0 = lane / D, t0 = lane; k0 < maxnb; k0 += kPasses * NPP, t0 += kPasses * LA) {
+      int32_t c[kPasses][R];
+      T v[kPasses][R][D], xv[kPasses][R];
 #pragma unroll
-      for (int r = 0; r < R; ++r) c[r] = k < nb[r] ? __ldg(S.nbr + p0[r] + k) : -1;
-      T v[R][D];
+      for (int u = 0; u < kPasses; ++u)
 #pragma unroll
-      for (int r = 0; r < R; ++r)
+        for (int r = 0; r < R; ++r) {
+          const int32_t k = k0 + u * NPP;
+          const bool in = k < nb[r];
+          c[u][r] = in ? __ldg(S.nbr + p0[r] + k) : -1;
 #pragma unroll
-        for (int i = 0; i < D; ++i)
-          v[r][i] = c[r] >= 0 ? __ldg(S.vals + (int64_t)D * D * p0[r] + (int64_t)i * D * nb[r] + t) : (T)0;
-      T xv[R];
+          for (int i = 0; i < D; ++i)
+            v[u][r][i] =
+                in ? __ldg(S.vals + (int64_t)D * D * p0[r] + (int64_t)i * D * nb[r] + t0 + u * LA) : (T)0;
+        }
 #pragma unroll
-      for (int r = 0; r < R; ++r) {
-        const T x = c[r] >= 0 ? xf((int64_t)c[r] * D + j) : (T)0;
-        xv[r] = DIFF && c[r] >= 0 ? x - self[r] : x;
-      }
+      for (int u = 0; u < kPasses; ++u)
 #pragma unroll
-      for (int r = 0; r < R; ++r)
+        for (int r = 0; r < R; ++r) {
+          const T x = c[u][r] >= 0 ? xf((int64_t)c[u][r] * D + j) : (T)0;
+          xv[u][r] = DIFF && c[u][r] >= 0 ? x - self[r] : x;
+        }
 #pragma unroll
-        for (int i = 0; i < D; ++i) acc[r][i] += v[r][i] * xv[r];
+      for (int u = 0; u < kPasses; ++u)
+#pragma unroll
+        for (int r = 0; r < R; ++r)
+#pragma unroll
+          for (int i = 0; i < D; ++i) acc[r][i] += v[u][r][i] * xv[u][r];
     }
   }
 #pragma unroll
@@ -214,7 +316,7 @@ __device__ __forceinline__ void node_rows_multi(const int64_t (&a)[R], int lane,
 // butterfly), ec = A_c^-1 rc (one warp per row; FP32 inverse for the FP32
 // iteration).  Every thread of the cluster calls it; r must be written.
 template <int D, typename T>
-__device__ void coarse_correct(Ctx& c, const gfea_batch_instance& I, const T* r, int64_t gtid, int64_t nthr) {
+__device__ __noinline__ void coarse_correct(Ctx& c, const gfea_batch_instance& I, const T* r, int64_t gtid, int64_t nthr) {
   constexpr int nr = Modes<D>::nr;
   const gfea_coarse_level& L = I.coarse;
   const int lane = threadIdx.x & 31;
@@ -226,15 +328,33 @@ __device__ void coarse_correct(Ctx& c, const gfea_batch_instance& I, const T* r,
 #pragma unroll
     for (int m = 0; m < nr; ++m) v[m] = 0;
     const int32_t k1 = L.agg_ptr[g + 1];
-    for (int32_t k = L.agg_ptr[g] + lane; k < k1; k += 32) {
-      const int64_t a = L.agg_nodes[k];
-      T R[D][nr];
-      node_modes<D, T>(off[a], I.known + a * D, R);
+    constexpr int B = D < 3 ? 4 : 2;  // nodes per lane with their loads in flight
+    for (int32_t k = L.agg_ptr[g] + lane; k < k1; k += B * 32) {
+      int64_t a[B];
+      T ri[B][D];
+      float4 o[B];
+      uint8_t kn[B][D];
 #pragma unroll
-      for (int i = 0; i < D; ++i) {
-        const T ri = ldcg(r + a * D + i);
+      for (int q = 0; q < B; ++q) a[q] = k + q * 32 < k1 ? L.agg_nodes[k + q * 32] : -1;
 #pragma unroll
-        for (int m = 0; m < nr; ++m) v[m] += R[i][m] * ri;
+      for (int q = 0; q < B; ++q) {
+        if (a[q] < 0) continue;
+        o[q] = off[a[q]];
+#pragma unroll
+        for (int i = 0; i < D; ++i) {
+          kn[q][i] = I.known[a[q] * D + i];
+          ri[q][i] = ldcg(r + a[q] * D + i);
+        }
+      }
+#pragma unroll
+      for (int q = 0; q < B; ++q) {
+        if (a[q] < 0) continue;
+        T R[D][nr];
+        node_modes<D, T>(o[q], kn[q], R);
+#pragma unroll
+        for (int i = 0; i < D; ++i)
+#pragma unroll
+          for (int m = 0; m < nr; ++m) v[m] += R[i][m] * ri[q][i];
       }
     }
 #pragma unroll
@@ -246,50 +366,90 @@ __device__ void coarse_correct(Ctx& c, const gfea_batch_instance& I, const T* r,
   }
   c.cl.sync();  // rc complete
   const int nc = L.nc;
-  for (int64_t i = gw; i < nc; i += nw) {
-    T acc = 0;
-    if (sizeof(T) == 4) {
-      const float* row = L.inv32 + i * nc;
-      for (int j = lane; j < nc; j += 32) acc += (T)__ldg(row + j) * (T)ldcg(L.rc + j);
-    } else {
-      const double* row = L.inv + i * nc;
-      for (int j = lane; j < nc; j += 32) acc += (T)(__ldg(row + j) * ldcg(L.rc + j));
+  constexpr int RG = 4;  // rows per warp with their loads in flight
+  for (int64_t i0 = gw; i0 < nc; i0 += RG * nw) {
+    int64_t row[RG];
+    T acc[RG];
+#pragma unroll
+    for (int q = 0; q < RG; ++q) {
+      row[q] = i0 + q * nw < nc ? i0 + q * nw : i0;
+      acc[q] = 0;
+    }
+    constexpr int U = sizeof(T) == 4 ? 6 : 3;
+    for (int j0 = lane; j0 < nc; j0 += 32 * U) {
+      T rj[U], ij[U][RG];
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const int j = j0 + 32 * u;
+        rj[u] = j < nc ? (T)ldcg(L.rc + j) : (T)0;
+#pragma unroll
+        for (int q = 0; q < RG; ++q)
+          ij[u][q] = j >= nc ? (T)0
+                             : (sizeof(T) == 4 ? (T)__ldg(L.inv32 + row[q] * nc + j) : (T)__ldg(L.inv + row[q] * nc + j));
+      }
+#pragma unroll
+      for (int u = 0; u < U; ++u)
+#pragma unroll
+        for (int q = 0; q < RG; ++q) acc[q] += ij[u][q] * rj[u];
     }
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-    if (lane == 0) L.ec[i] = (double)acc;
+    for (int q = 0; q < RG; ++q) {
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) acc[q] += __shfl_xor_sync(0xffffffffu, acc[q], o);
+      if (lane == 0 && i0 + q * nw < nc) L.ec[i0 + q * nw] = (double)acc[q];
+    }
   }
   c.cl.sync();  // ec complete
 }
 
 // z = D^-1 r + R ec[agg] (masked) for the nodes of this thread; partials r.z, r.r.
 template <int D, typename T>
-__device__ void z_two_level(const gfea_batch_instance& I, const BatchBuf<T>& w, int64_t gtid, int64_t nthr,
+__device__ __noinline__ void z_two_level(const gfea_batch_instance& I, const BatchBuf<T>& w, int64_t gtid, int64_t nthr,
                             DotAcc<T>& rz, DotAcc<T>& rr) {
   constexpr int nr = Modes<D>::nr;
   const gfea_coarse_level& L = I.coarse;
   const float4* off = reinterpret_cast<const float4*>(L.off);
-  for (int64_t a = gtid; a < I.n_nodes; a += nthr) {
-    T rl[D];
+  constexpr int B = D * sizeof(T) <= 8 ? 4 : (D * sizeof(T) <= 12 ? 2 : 1);  // nodes per thread with their loads in flight
+  for (int64_t a0 = gtid; a0 < I.n_nodes; a0 += B * nthr) {
+    T rl[B][D], di[B][D][D], e[B][nr];
+    float4 o[B];
+    uint8_t kn[B][D];
+    int g[B];
 #pragma unroll
-    for (int i = 0; i < D; ++i) rl[i] = ldcg(w.r + a * D + i);
-    const int g = L.agg[a];
-    T R[D][nr];
-    node_modes<D, T>(off[a], I.known + a * D, R);
-    T e[nr];
+    for (int q = 0; q < B; ++q) {
+      const int64_t a = a0 + q * nthr < I.n_nodes ? a0 + q * nthr : a0;
+      g[q] = L.agg[a];
+      o[q] = off[a];
 #pragma unroll
-    for (int m = 0; m < nr; ++m) e[m] = (T)ldcg(L.ec + g * nr + m);
+      for (int i = 0; i < D; ++i) {
+        rl[q][i] = ldcg(w.r + a * D + i);
+        kn[q][i] = I.known[a * D + i];
 #pragma unroll
-    for (int i = 0; i < D; ++i) {
-      T zi = 0;
+        for (int j = 0; j < D; ++j) di[q][i][j] = w.dinv[a * D * D + i * D + j];
+      }
+    }
 #pragma unroll
-      for (int j = 0; j < D; ++j) zi += w.dinv[a * D * D + i * D + j] * rl[j];
+    for (int q = 0; q < B; ++q)
 #pragma unroll
-      for (int m = 0; m < nr; ++m) zi += R[i][m] * e[m];
-      if (I.known[a * D + i]) zi = 0;
-      w.z[a * D + i] = zi;
-      rz.add_prod(rl[i], zi);
-      rr.add_prod(rl[i], rl[i]);
+      for (int m = 0; m < nr; ++m) e[q][m] = (T)ldcg(L.ec + g[q] * nr + m);
+#pragma unroll
+    for (int q = 0; q < B; ++q) {
+      const int64_t a = a0 + q * nthr;
+      if (a >= I.n_nodes) break;
+      T R[D][nr];
+      node_modes<D, T>(o[q], kn[q], R);
+#pragma unroll
+      for (int i = 0; i < D; ++i) {
+        T zi = 0;
+#pragma unroll
+        for (int j = 0; j < D; ++j) zi += di[q][i][j] * rl[q][j];
+#pragma unroll
+        for (int m = 0; m < nr; ++m) zi += R[i][m] * e[q][m];
+        if (kn[q][i]) zi = 0;
+        w.z[a * D + i] = zi;
+        rz.add_prod(rl[q][i], zi);
+        rr.add_prod(rl[q][i], rl[q][i]);
+      }
     }
   }
 }
@@ -308,6 +468,62 @@ __device__ void restart_rz_two_level(Ctx& c, const gfea_batch_instance& I, const
   v[1] = rr.value();
 }
 
+// Direction pb = z + beta pa and Ap = A pb (masked SpMV); this thread's partial
+// of pb.Ap.
+template <int D, int G, typename T, bool DIFF>
+__device__ __noinline__ double direction_apply(const SysT<T>& S, const T* z, const T* pa, T* pb, T* Ap, T beta,
+                                               int64_t grp, int64_t ngrp, int lane) {
+  const int64_t Nn = S.Nn;
+  const int64_t sub = grp % (32 / G);
+  DotAcc<T> pap;
+  constexpr int R = D * sizeof(T) <= 12 ? 4 : 2;  // rows per group per round
+  // the row pointers of the next round are fetched during this one
+  int32_t q0[R], q1[R];
+  auto fetch = [&](int64_t a0) {
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      const int64_t a = a0 + sub + (int64_t)r * ngrp;
+      const int64_t ac = a < Nn ? a : Nn - 1;
+      q0[r] = __ldg(S.node_ptr + ac);
+      q1[r] = __ldg(S.node_ptr + ac + 1);
+    }
+  };
+  fetch(grp - sub);
+  for (int64_t a0 = grp - sub; a0 < Nn; a0 += (int64_t)R * ngrp) {
+    int64_t an[R], ac[R];
+    int32_t p0[R], nb[R];
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      an[r] = a0 + sub + (int64_t)r * ngrp;
+      ac[r] = an[r] < Nn ? an[r] : Nn - 1;
+      p0[r] = q0[r];
+      nb[r] = q1[r] - q0[r];
+    }
+    fetch(a0 + (int64_t)R * ngrp);
+    uint8_t kn[R];
+#pragma unroll
+    for (int r = 0; r < R; ++r) kn[r] = S.known[ac[r] * D + lane % D];
+    T acc[R][D], self[R];
+    auto dir = [&](int64_t cc) { return ldcg(z + cc) + beta * ldcg(pa + cc); };
+    node_rows_multi<D, G, T, DIFF, R>(ac, p0, nb, lane, S, dir, acc, self);
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      if (an[r] < Nn && lane < D) {
+        T av = acc[r][0];
+#pragma unroll
+        for (int i = 1; i < D; ++i)
+          if (lane == i) av = acc[r][i];
+        const int64_t dof = an[r] * D + lane;
+        if (kn[r]) av = 0;
+        pb[dof] = self[r];
+        Ap[dof] = av;
+        pap.add_prod(self[r], av);
+      }
+    }
+  }
+  return pap.value();
+}
+
 template <int D, int G, typename T>
 __device__ void solve_instance(Ctx& c, const gfea_batch_instance& I, double delta2) {
   const int64_t Nn = I.n_nodes;
@@ -317,8 +533,8 @@ __device__ void solve_instance(Ctx& c, const gfea_batch_instance& I, double delt
   const SysT<T> S{Nn, I.node_ptr, I.nbr, vals, I.known, I.translation_invariant};
   const SysT<double> S64{Nn, I.node_ptr, I.nbr, I.vals64, I.known, 0};
   const int tid = threadIdx.x;
-  const int64_t gtid = (int64_t)c.rank * kBT + tid;
-  const int64_t nthr = (int64_t)kCL * kBT;
+  const int64_t gtid = (int64_t)c.rank * blockDim.x + tid;
+  const int64_t nthr = (int64_t)kCL * blockDim.x;
   const int lane = tid % G;
   const int64_t grp = gtid / G, ngrp = nthr / G;
   const int64_t sub = grp % (32 / G);
@@ -410,41 +626,9 @@ __device__ void solve_instance(Ctx& c, const gfea_batch_instance& I, double delt
     T* pb = w.pb;
     const bool diff = sizeof(T) == 4 && S.diff;
     for (;;) {
-      // direction p' = z + beta p and Ap' (masked SpMV); partial p'.Ap'
-      double va[1] = {0}, oa[1];
-      DotAcc<T> pap_acc;
-      const T bt = (T)beta;
-      constexpr int R = 4;  // rows per group per round
-      for (int64_t a0 = grp - sub; a0 < Nn; a0 += (int64_t)R * ngrp) {
-        int64_t an[R], ac[R];
-#pragma unroll
-        for (int r = 0; r < R; ++r) {
-          an[r] = a0 + sub + (int64_t)r * ngrp;
-          ac[r] = an[r] < Nn ? an[r] : Nn - 1;
-        }
-        T acc[R][D];
-        auto dir = [&](int64_t cc) { return ldcg(w.z + cc) + bt * ldcg(pa + cc); };
-        if (diff)
-          node_rows_multi<D, G, T, true, R>(ac, lane, S, dir, acc);
-        else
-          node_rows_multi<D, G, T, false, R>(ac, lane, S, dir, acc);
-#pragma unroll
-        for (int r = 0; r < R; ++r) {
-          if (an[r] < Nn && lane < D) {
-            T av = acc[r][0];
-#pragma unroll
-            for (int i = 1; i < D; ++i)
-              if (lane == i) av = acc[r][i];
-            const int64_t dof = an[r] * D + lane;
-            const T pn = ldcg(w.z + dof) + bt * ldcg(pa + dof);
-            if (S.known[dof]) av = 0;
-            pb[dof] = pn;
-            w.Ap[dof] = av;
-            pap_acc.add_prod(pn, av);
-          }
-        }
-      }
-      va[0] = pap_acc.value();
+      double va[1], oa[1];
+      va[0] = diff ? direction_apply<D, G, T, true>(S, w.z, pa, pb, w.Ap, (T)beta, grp, ngrp, lane)
+                   : direction_apply<D, G, T, false>(S, w.z, pa, pb, w.Ap, (T)beta, grp, ngrp, lane);
       csum<1>(c, va, oa);
       const double pap = oa[0];
       if (!(pap > 0) || !isfinite(pap)) {
@@ -457,13 +641,27 @@ __device__ void solve_instance(Ctx& c, const gfea_batch_instance& I, double delt
       DotAcc<T> rz_acc, rr_acc;
       const T al = (T)alpha;
       if (two_level) {  // x, r; then the coarse correction; then z
-        for (int64_t a = gtid; a < Nn; a += nthr)
+        constexpr int B = 4;  // unknowns per thread with their loads in flight
+        const int64_t N = Nn * D;
+        for (int64_t d0 = gtid; d0 < N; d0 += B * nthr) {
+          T xo[B], po[B], ro[B], ao[B];
 #pragma unroll
-          for (int i = 0; i < D; ++i) {
-            const int64_t dof = a * D + i;
-            w.dx[dof] = ldcg(w.dx + dof) + al * ldcg(pb + dof);
-            w.r[dof] = ldcg(w.r + dof) - al * ldcg(w.Ap + dof);
+          for (int q = 0; q < B; ++q) {
+            const int64_t dof = d0 + q * nthr < N ? d0 + q * nthr : d0;
+            xo[q] = ldcg(w.dx + dof);
+            po[q] = ldcg(pb + dof);
+            ro[q] = ldcg(w.r + dof);
+            ao[q] = ldcg(w.Ap + dof);
           }
+#pragma unroll
+          for (int q = 0; q < B; ++q) {
+            const int64_t dof = d0 + q * nthr;
+            if (dof < N) {
+              w.dx[dof] = xo[q] + al * po[q];
+              w.r[dof] = ro[q] - al * ao[q];
+            }
+          }
+        }
         coarse_correct<D, T>(c, I, w.r, gtid, nthr);
         z_two_level<D, T>(I, w, gtid, nthr, rz_acc, rr_acc);
       } else
@@ -561,25 +759,59 @@ __device__ void dispatch(Ctx& c, const gfea_batch_instance& I, double delta2) {
   }
 }
 
-__global__ void __cluster_dims__(kCL, 1, 1) __launch_bounds__(kBT, 2)
-    batch_pcg_kernel(const gfea_batch_instance* __restrict__ insts, int n, int* next, int fp64, double delta2) {
+// One launch per width; the systems are sorted by stored values, the wide ones
+// first.  The narrow launch is a programmatic dependent of the wide one: it
+// starts when the wide clusters hold their SMs, takes the SMs they leave, and
+// completes after them.
+template <typename T, int BT>
+__global__ void __cluster_dims__(kCL, 1, 1) __launch_bounds__(BT, 2 * kNarrow / BT)
+    batch_pcg_kernel(const gfea_batch_instance* __restrict__ insts, int n, int* next, double delta2) {
   __shared__ double slots[8];
-  __shared__ double sh[32];
+  __shared__ double sh[4 * (kWide / 32)];
   __shared__ int s_idx;
+  if (BT == kWide) cudaTriggerProgrammaticLaunchCompletion();
   Ctx c{cg::this_cluster(), 0, slots, sh, 0};
   c.rank = c.cl.block_rank();
+  int split = 0, hi = n;  // the wide systems are [0, split)
+  while (split < hi) {
+    const int mid = (split + hi) >> 1;
+    if (stored_values(insts[mid]) >= kWideValues) split = mid + 1; else hi = mid;
+  }
+  const int first = BT == kWide ? 0 : split, last = BT == kWide ? split : n;
   for (;;) {
-    if (c.rank == 0 && threadIdx.x == 0) s_idx = atomicAdd(next, 1);
+    if (c.rank == 0 && threadIdx.x == 0) s_idx = first + atomicAdd(next + (BT == kWide ? 0 : 1), 1);
     c.cl.sync();
     const int idx = *c.cl.map_shared_rank(&s_idx, 0);
     c.cl.sync();  // rank 0's slot is read by all before it changes
-    if (idx >= n) break;
+    if (idx >= last) break;
     const gfea_batch_instance I = insts[idx];
-    if (fp64)
-      dispatch<double>(c, I, 1e-6);
-    else
-      dispatch<float>(c, I, delta2);
+    dispatch<T>(c, I, delta2);
   }
+  if (BT == kNarrow) cudaGridDependencySynchronize();
+}
+
+// Persistent clusters: enough to fill the GPU, never more than the systems.
+// The wide launch takes no more than can be resident at once, so that the
+// narrow one does not wait for a wide solve to end.
+template <typename T>
+int launch_widths(const gfea_batch_instance* desc, int n, int* next, double delta2, cudaStream_t s) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.stream = s;
+  cfg.blockDim = dim3(kWide);
+  cfg.gridDim = dim3(kCL);
+  int resident = 0;
+  GFEA_CUDA_TRY(cudaOccupancyMaxActiveClusters(&resident, batch_pcg_kernel<T, kWide>, &cfg));
+  cfg.gridDim = dim3(kCL * std::max(1, std::min(n, resident)));
+  GFEA_CUDA_TRY(cudaLaunchKernelEx(&cfg, batch_pcg_kernel<T, kWide>, desc, n, next, delta2));
+  cudaLaunchAttribute overlap = {};
+  overlap.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  overlap.val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = &overlap;
+  cfg.numAttrs = 1;
+  cfg.blockDim = dim3(kNarrow);
+  cfg.gridDim = dim3(kCL * std::max(1, std::min(n, 2 * kSMs / kCL)));
+  GFEA_CUDA_TRY(cudaLaunchKernelEx(&cfg, batch_pcg_kernel<T, kNarrow>, desc, n, next, delta2));
+  return GFEA_OK;
 }
 
 }  // namespace
@@ -624,7 +856,7 @@ extern "C" int gfea_batch_prepare(const gfea_batch_instance* inst_host, int n, v
   // largest systems first (longest-processing-time order over the clusters)
   std::vector<gfea_batch_instance> order(inst_host, inst_host + n);
   std::stable_sort(order.begin(), order.end(), [](const gfea_batch_instance& a, const gfea_batch_instance& b) {
-    return a.n_pairs * a.dof_n * a.dof_n > b.n_pairs * b.dof_n * b.dof_n;
+    return stored_values(a) > stored_values(b);
   });
   auto* desc = reinterpret_cast<gfea_batch_instance*>(static_cast<char*>(scratch) + a256(sizeof(int)));
   GFEA_CUDA_TRY(cudaMemcpyAsync(desc, order.data(), sizeof(gfea_batch_instance) * (size_t)n, cudaMemcpyHostToDevice,
@@ -642,14 +874,9 @@ extern "C" int gfea_batch_launch(void* scratch, int n, const gfea_pcg_opts* opts
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   int* next = static_cast<int*>(scratch);
   auto* desc = reinterpret_cast<gfea_batch_instance*>(static_cast<char*>(scratch) + a256(sizeof(int)));
-  GFEA_CUDA_TRY(cudaMemsetAsync(next, 0, sizeof(int), s));
-  // persistent clusters: enough to fill the GPU, never more than the systems
-  int clusters = std::min(n, 2 * kSMs / kCL);
-  if (clusters < 1) clusters = 1;
+  GFEA_CUDA_TRY(cudaMemsetAsync(next, 0, 2 * sizeof(int), s));
   const double d = (opts_host->inner_rtol > 0 && opts_host->inner_rtol < 1) ? opts_host->inner_rtol : 0.1;
-  batch_pcg_kernel<<<clusters * kCL, kBT, 0, s>>>(desc, n, next, prec == GFEA_F64 ? 1 : 0, d * d);
-  GFEA_LAUNCH_CHECK();
-  return GFEA_OK;
+  return prec == GFEA_F64 ? launch_widths<double>(desc, n, next, 1e-6, s) : launch_widths<float>(desc, n, next, d * d, s);
 }
 
 extern "C" int gfea_batch_pcg(const gfea_batch_instance* inst_host, int n, void* scratch, size_t scratch_bytes,
