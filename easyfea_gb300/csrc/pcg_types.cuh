@@ -21,7 +21,7 @@ struct CoarseHdr {
 // (block b adds into copy b % kRcCopies): one copy held them all on a few L2
 // slices, where they serialised.  Below kRcCopyMinNodes nodes the atomics
 // are few and an iteration is launch-latency bound: one copy (rc itself,
-// cleared by finish_z) and no summing launch.
+// cleared by the coarse solve) and no summing launch.
 constexpr int kRcCopies = 16;
 constexpr int64_t kRcCopyMinNodes = 100000;
 
@@ -33,7 +33,7 @@ struct CoarseDev {
   float4* off = nullptr;   // node offset from its cell centre / largest cell size
   double* Ac = nullptr;    // nc x nc, inverted in place
   // working storage of the inversion: float-float pairs (hi, lo)
-  float* Ahi = nullptr;    // nc x nc
+  float* Ahi = nullptr;    // nc x nc (batched inversion)
   float* Alo = nullptr;
   float* rowph = nullptr;  // kGJB x nc: row panel of the pivot block
   float* rowpl = nullptr;

@@ -1358,8 +1358,6 @@ size_t pcg_layout(int64_t Nn, int D, int n_agg_max, PcgWork* w, char* base, size
     w->C.agg = reinterpret_cast<int32_t*>(take(sizeof(int32_t) * Nn));
     w->C.off = reinterpret_cast<float4*>(take(sizeof(float4) * Nn));
     w->C.Ac = reinterpret_cast<double*>(take(sizeof(double) * nc * nc));
-    w->C.Ahi = reinterpret_cast<float*>(take(sizeof(float) * nc * nc));
-    w->C.Alo = reinterpret_cast<float*>(take(sizeof(float) * nc * nc));
     w->C.rowph = reinterpret_cast<float*>(take(sizeof(float) * kGJB * nc));
     w->C.rowpl = reinterpret_cast<float*>(take(sizeof(float) * kGJB * nc));
     w->C.colph = reinterpret_cast<float*>(take(sizeof(float) * kGJB * nc));
