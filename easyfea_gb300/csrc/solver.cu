@@ -780,29 +780,35 @@ __global__ void __launch_bounds__(kThreads) rc_sum_kernel(CoarseDev C, const Sca
   }
 }
 
-// ec = A_c^-1 rc: one block of kGemvThreads per coarse row (enough warps in
-// flight to stream the L2-resident inverse), fixed-order block reduction.
-constexpr int kGemvThreads = 128;
-
-// The last block to finish completes r.z = r.y + rc.ec, derives beta and the
-// convergence state exactly as update_kernel does, and clears a single-copy
-// rc for the next restriction.
-__global__ void __launch_bounds__(kGemvThreads) coarse_gemv_kernel(CoarseDev C, double* partials, Scal* sc, int mode) {
+// ec = A_c^-1 rc: kGemvThreads threads per coarse row (enough warps in flight
+// to stream the L2-resident inverse), kGemvRows rows per block, fixed-order
+// row sums.  rc.ec, which completes r.z, is summed by the last block, so
+// blocks of several rows: with one row a block, the 1,152 tickets and
+// partials of the 2.02M-unknown box's coarse level took a third of the kernel
+// (16.9 us one row a block, 13.7 us four).
+constexpr int kGemvThreads = 128, kGemvRows = 4;
+__global__ void __launch_bounds__(kGemvThreads* kGemvRows)
+    coarse_gemv_kernel(CoarseDev C, double* partials, Scal* sc, int mode) {
   if (mode == 0 && sc->done) return;
-  __shared__ double sh[kGemvThreads / 32];
+  constexpr int kWarps = kGemvThreads / 32;  // warps per row
+  __shared__ double sh[kGemvRows * kWarps];
+  const int sub = threadIdx.x / kGemvThreads, t0 = threadIdx.x % kGemvThreads;
   double dot[1] = {0};
-  for (int i = blockIdx.x; i < C.nc; i += gridDim.x) {
-    const double* row = C.Ac + (int64_t)i * C.nc;
+  for (int i0 = blockIdx.x * kGemvRows; i0 < C.nc; i0 += gridDim.x * kGemvRows) {
+    const int i = i0 + sub;
     double v = 0;
-    for (int j = threadIdx.x; j < C.nc; j += kGemvThreads) v += row[j] * C.rc[j];
+    if (i < C.nc) {
+      const double* row = C.Ac + (int64_t)i * C.nc;
+      for (int j = t0; j < C.nc; j += kGemvThreads) v += row[j] * C.rc[j];
+    }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
     if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = v;
     __syncthreads();
-    if (threadIdx.x == 0) {
+    if (t0 == 0 && i < C.nc) {
       double t = 0;
 #pragma unroll
-      for (int w = 0; w < kGemvThreads / 32; ++w) t += sh[w];
+      for (int w = 0; w < kWarps; ++w) t += sh[sub * kWarps + w];
       C.ec[i] = t;
       C.ecf[i] = (float)t;
       dot[0] += t * C.rc[i];
@@ -1631,7 +1637,8 @@ int launch_precond(const gfea_system* s, PcgWork& w, T* x, T* p, int mode, cudaS
     rc_sum_kernel<<<(int)ceil_div(w.C.nc, kThreads), kThreads, 0, st>>>(w.C, w.sc, mode);
     GFEA_LAUNCH_CHECK();
   }
-  coarse_gemv_kernel<<<std::min(w.C.nc, 8 * kSMs), kGemvThreads, 0, st>>>(w.C, w.partials, w.sc, mode);
+  coarse_gemv_kernel<<<(int)std::min<int64_t>(ceil_div(w.C.nc, kGemvRows), 8 * kSMs), kGemvThreads * kGemvRows, 0, st>>>(
+      w.C, w.partials, w.sc, mode);
   GFEA_LAUNCH_CHECK();
   e = prof_mark(st, kTagGemv);
   if (e) return e;
