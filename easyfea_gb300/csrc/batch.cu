@@ -16,7 +16,7 @@
 // of 2000 to 50000 unknowns, mixed precision, assembly included: 26.8 ms with
 // one neighbour pass and one node at a time and 256 threads throughout, 23.9
 // with the batched loads, 16.8 with the wide clusters; 64 of 3000 unknowns
-// 9.2 -> 6.9 ms.
+// 9.2 -> 7.3 ms, 256 of 2000 to 200000 276 -> 228 ms.
 //
 // Cross-CTA reads of vectors written inside the launch use L2-only loads
 // (ld.global.cg), so no stale L1 line is ever consulted; the cluster barrier
@@ -39,14 +39,21 @@ namespace {
 
 constexpr int kCL = 8;    // CTAs per cluster (portable cluster size)
 
-// Threads per CTA: 256 (two CTAs per SM), or 512 (one) for the systems of at
-// least kWideValues stored values.  A cluster's passes over its rows are bound
-// by L2 latency at either width, so twice the warps shorten a solve (24021
-// QUAD4 nodes: 19.0 -> 14.4 ms, 5425: 5.4 -> 4.8 ms) for twice the SMs: worth
-// it where a large system is the tail of the launch, not for many small ones
-// (64 systems of 3000 unknowns: 6.9 ms narrow, 13.3 ms wide; 40 of 20000:
-// 24.9 and 27.0).  The width follows the system's own size alone, so its
-// result does not depend on the others in the launch.
+// Threads per CTA: 256 (two CTAs per SM), or 512 (one) for systems of at least
+// kWideValues stored values where they are the tail of their batch.  A
+// cluster's passes over its rows are bound by L2 latency at either width, so
+// twice the warps shorten a solve (24021 QUAD4 nodes: 19.0 -> 14.4 ms, 5425:
+// 5.4 -> 4.8 ms), but 8 whole SMs a cluster leave SMs unused and small systems
+// wait on barriers.  2000 to 50000 unknowns, 32 systems: 22.0 ms narrow, 16.2
+// wide; to 60000, 40 systems: 29.7 and 20.3, 100 systems: 40.0 and 43.2; 64 of
+// 3000: 7.3 and 13.3; 256 of 2000 to 200000: 228 and 280.  So: wide where the
+// largest system is over twice its share of the batch (the time of the batch
+// on all narrow clusters).
+//
+// Both widths divide a system among the same kCL * 512 virtual threads, of
+// which a thread of the narrow one is two (VT, kWide / VT apart), and sum
+// their partials in the same order: a system's result is the same to the bit
+// at either width, so it does not depend on the others in the launch.
 constexpr int kNarrow = 256, kWide = 512;
 constexpr int64_t kWideValues = 400000;
 
@@ -95,27 +102,30 @@ struct Ctx {
   int phase;
 };
 
-// Cluster-wide sum of NV values; every thread of every CTA gets the same result.
+// Cluster-wide sum of NV values (one per virtual thread); every thread of every
+// CTA gets the same result.
 // (c.sh is free again once the cluster barrier has been passed.)
-template <int NV>
-__device__ void csum(Ctx& c, const double (&v)[NV], double (&out)[NV]) {
-  const int warps = blockDim.x >> 5;
+template <int NV, int VT>
+__device__ void csum(Ctx& c, const double (&v)[VT][NV], double (&out)[NV]) {
+  constexpr int kWarps = kWide / 32;
   double* slot = c.slots + (c.phase & 1) * 4;
   const int wp = threadIdx.x >> 5, l = threadIdx.x & 31;
 #pragma unroll
-  for (int k = 0; k < NV; ++k) {
-    double t = v[k];
+  for (int k = 0; k < NV; ++k)
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
-    if (l == 0) c.sh[k * (kWide / 32) + wp] = t;
-  }
+    for (int q = 0; q < VT; ++q) {
+      double t = v[q][k];
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+      if (l == 0) c.sh[k * kWarps + q * (kWarps / VT) + wp] = t;
+    }
   __syncthreads();
   if (wp == 0) {
 #pragma unroll
     for (int k = 0; k < NV; ++k) {
-      double t = l < warps ? c.sh[k * (kWide / 32) + l] : 0.0;
+      double t = l < kWarps ? c.sh[k * kWarps + l] : 0.0;
 #pragma unroll
-      for (int o = kWide / 64; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+      for (int o = kWarps / 2; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
       if (l == 0) slot[k] = t;
     }
   }
@@ -139,23 +149,23 @@ __device__ void csum(Ctx& c, const double (&v)[NV], double (&out)[NV]) {
 // trips, as node_rows_multi below).
 constexpr int kPasses = 3;
 
-template <int D, int G>
+template <int D, int G, int VT>
 __device__ __noinline__ void resid64(const SysT<double>& S, const double* b, const double* x, double* r64, int64_t grp,
-                        int64_t ngrp, int lane, double (&v)[4]) {
+                                     int64_t ngrp, int lane, double (&v)[VT][4]) {
   constexpr int LA = G - G % D;
   constexpr int NPP = LA / D;
-  constexpr int R = D < 3 ? 2 : 1;
+  constexpr int R = D < 3 || VT == 2 ? 2 : 1;
   const int64_t Nn = S.Nn;
   const int64_t sub = grp % (32 / G);
   const int j = lane % D;
-  for (int64_t a0 = grp - sub; a0 < Nn; a0 += R * ngrp) {
+  for (int64_t a0 = grp - sub; a0 < Nn; a0 += (R / VT) * ngrp) {
     int64_t an[R];
     int32_t p0[R], nb[R];
     double all[R][D], kn[R][D], ab[R][D];
     int32_t maxnb = 0;
 #pragma unroll
     for (int r = 0; r < R; ++r) {
-      an[r] = a0 + sub + r * ngrp;
+      an[r] = a0 + sub + (r % VT) * (kWide / VT / G) + (r / VT) * ngrp;
       const int64_t ac = an[r] < Nn ? an[r] : Nn - 1;
       p0[r] = S.node_ptr[ac];
       nb[r] = S.node_ptr[ac + 1] - p0[r];
@@ -218,9 +228,9 @@ __device__ __noinline__ void resid64(const SysT<double>& S, const double* b, con
           const double rci = unk ? bi - kn[r][i] : 0.0;
           const double ai = unk ? ab[r][i] + fabs(bi) : 0.0;
           r64[dof] = ri;
-          v[0] += ri * ri;
-          v[1] += rci * rci;
-          v[2] += ai * ai;
+          v[r % VT][0] += ri * ri;
+          v[r % VT][1] += rci * rci;
+          v[r % VT][2] += ai * ai;
         }
       }
     }
@@ -228,28 +238,30 @@ __device__ __noinline__ void resid64(const SysT<double>& S, const double* b, con
 }
 
 // r = (T) r64, z = D^-1 r (masked) for the nodes of this thread; partials r.z, r.r.
-template <int D, typename T>
+template <int D, typename T, int VT>
 __device__ void restart_rz(const gfea_batch_instance& I, const BatchBuf<T>& w, int64_t gtid, int64_t nthr,
-                           double (&v)[2]) {
-  for (int64_t a = gtid; a < I.n_nodes; a += nthr) {
-    T rl[D];
+                           double (&v)[VT][2]) {
 #pragma unroll
-    for (int i = 0; i < D; ++i) {
-      const int64_t dof = a * D + i;
-      rl[i] = (T)ldcg(w.r64 + dof);
-      w.r[dof] = rl[i];
+  for (int q = 0; q < VT; ++q)
+    for (int64_t a = gtid + q * (kWide / VT); a < I.n_nodes; a += nthr) {
+      T rl[D];
+#pragma unroll
+      for (int i = 0; i < D; ++i) {
+        const int64_t dof = a * D + i;
+        rl[i] = (T)ldcg(w.r64 + dof);
+        w.r[dof] = rl[i];
+      }
+#pragma unroll
+      for (int i = 0; i < D; ++i) {
+        T zi = 0;
+#pragma unroll
+        for (int j = 0; j < D; ++j) zi += ldcg(w.dinv + a * D * D + i * D + j) * rl[j];
+        if (I.known[a * D + i]) zi = 0;
+        w.z[a * D + i] = zi;
+        v[q][0] += (double)rl[i] * (double)zi;
+        v[q][1] += (double)rl[i] * (double)rl[i];
+      }
     }
-#pragma unroll
-    for (int i = 0; i < D; ++i) {
-      T zi = 0;
-#pragma unroll
-      for (int j = 0; j < D; ++j) zi += w.dinv[a * D * D + i * D + j] * rl[j];
-      if (I.known[a * D + i]) zi = 0;
-      w.z[a * D + i] = zi;
-      v[0] += (double)rl[i] * (double)zi;
-      v[1] += (double)rl[i] * (double)rl[i];
-    }
-  }
 }
 
 // node_rows for R nodes at once (one G-lane group): the index, value and
@@ -403,21 +415,23 @@ __device__ __noinline__ void coarse_correct(Ctx& c, const gfea_batch_instance& I
 }
 
 // z = D^-1 r + R ec[agg] (masked) for the nodes of this thread; partials r.z, r.r.
-template <int D, typename T>
+template <int D, typename T, int VT>
 __device__ __noinline__ void z_two_level(const gfea_batch_instance& I, const BatchBuf<T>& w, int64_t gtid, int64_t nthr,
-                            DotAcc<T>& rz, DotAcc<T>& rr) {
+                                         double (&out)[VT][2]) {
   constexpr int nr = Modes<D>::nr;
   const gfea_coarse_level& L = I.coarse;
   const float4* off = reinterpret_cast<const float4*>(L.off);
-  constexpr int B = D * sizeof(T) <= 8 ? 4 : (D * sizeof(T) <= 12 ? 2 : 1);  // nodes per thread with their loads in flight
-  for (int64_t a0 = gtid; a0 < I.n_nodes; a0 += B * nthr) {
+  constexpr int B = D * sizeof(T) <= 8 ? 4 : (D * sizeof(T) <= 12 ? 2 : VT);  // nodes per thread with their loads in flight
+  DotAcc<T> rz[VT], rr[VT];
+  for (int64_t a0 = gtid; a0 < I.n_nodes; a0 += (B / VT) * nthr) {
+    auto node = [&](int q) { return a0 + (q % VT) * (kWide / VT) + (q / VT) * nthr; };
     T rl[B][D], di[B][D][D], e[B][nr];
     float4 o[B];
     uint8_t kn[B][D];
     int g[B];
 #pragma unroll
     for (int q = 0; q < B; ++q) {
-      const int64_t a = a0 + q * nthr < I.n_nodes ? a0 + q * nthr : a0;
+      const int64_t a = node(q) < I.n_nodes ? node(q) : a0;
       g[q] = L.agg[a];
       o[q] = off[a];
 #pragma unroll
@@ -425,7 +439,7 @@ __device__ __noinline__ void z_two_level(const gfea_batch_instance& I, const Bat
         rl[q][i] = ldcg(w.r + a * D + i);
         kn[q][i] = I.known[a * D + i];
 #pragma unroll
-        for (int j = 0; j < D; ++j) di[q][i][j] = w.dinv[a * D * D + i * D + j];
+        for (int j = 0; j < D; ++j) di[q][i][j] = ldcg(w.dinv + a * D * D + i * D + j);
       }
     }
 #pragma unroll
@@ -434,8 +448,8 @@ __device__ __noinline__ void z_two_level(const gfea_batch_instance& I, const Bat
       for (int m = 0; m < nr; ++m) e[q][m] = (T)ldcg(L.ec + g[q] * nr + m);
 #pragma unroll
     for (int q = 0; q < B; ++q) {
-      const int64_t a = a0 + q * nthr;
-      if (a >= I.n_nodes) break;
+      const int64_t a = node(q);
+      if (a >= I.n_nodes) continue;
       T R[D][nr];
       node_modes<D, T>(o[q], kn[q], R);
 #pragma unroll
@@ -447,59 +461,63 @@ __device__ __noinline__ void z_two_level(const gfea_batch_instance& I, const Bat
         for (int m = 0; m < nr; ++m) zi += R[i][m] * e[q][m];
         if (kn[q][i]) zi = 0;
         w.z[a * D + i] = zi;
-        rz.add_prod(rl[q][i], zi);
-        rr.add_prod(rl[q][i], rl[q][i]);
+        rz[q % VT].add_prod(rl[q][i], zi);
+        rr[q % VT].add_prod(rl[q][i], rl[q][i]);
       }
     }
+  }
+#pragma unroll
+  for (int q = 0; q < VT; ++q) {
+    out[q][0] = rz[q].value();
+    out[q][1] = rr[q].value();
   }
 }
 
 // restart_rz with the coarse level: r = (T) r64, coarse correction, z.
-template <int D, typename T>
+template <int D, typename T, int VT>
 __device__ void restart_rz_two_level(Ctx& c, const gfea_batch_instance& I, const BatchBuf<T>& w, int64_t gtid,
-                                     int64_t nthr, double (&v)[2]) {
-  for (int64_t a = gtid; a < I.n_nodes; a += nthr)
+                                     int64_t nthr, double (&v)[VT][2]) {
+  const int64_t rtid = (int64_t)c.rank * blockDim.x + threadIdx.x, rthr = (int64_t)kCL * blockDim.x;
+  for (int64_t a = rtid; a < I.n_nodes; a += rthr)
 #pragma unroll
     for (int i = 0; i < D; ++i) w.r[a * D + i] = (T)ldcg(w.r64 + a * D + i);
-  coarse_correct<D, T>(c, I, w.r, gtid, nthr);
-  DotAcc<T> rz, rr;
-  z_two_level<D, T>(I, w, gtid, nthr, rz, rr);
-  v[0] = rz.value();
-  v[1] = rr.value();
+  coarse_correct<D, T>(c, I, w.r, rtid, rthr);
+  z_two_level<D, T, VT>(I, w, gtid, nthr, v);
 }
 
-// Direction pb = z + beta pa and Ap = A pb (masked SpMV); this thread's partial
-// of pb.Ap.
-template <int D, int G, typename T, bool DIFF>
-__device__ __noinline__ double direction_apply(const SysT<T>& S, const T* z, const T* pa, T* pb, T* Ap, T beta,
-                                               int64_t grp, int64_t ngrp, int lane) {
+// Direction pb = z + beta pa and Ap = A pb (masked SpMV); the partials of
+// pb.Ap.
+template <int D, int G, typename T, bool DIFF, int VT>
+__device__ __noinline__ void direction_apply(const SysT<T>& S, const T* z, const T* pa, T* pb, T* Ap, T beta,
+                                             int64_t grp, int64_t ngrp, int lane, double (&out)[VT][1]) {
   const int64_t Nn = S.Nn;
   const int64_t sub = grp % (32 / G);
-  DotAcc<T> pap;
+  DotAcc<T> pap[VT];
   constexpr int R = D * sizeof(T) <= 12 ? 4 : 2;  // rows per group per round
   // the row pointers of the next round are fetched during this one
   int32_t q0[R], q1[R];
+  auto row = [&](int64_t a0, int r) { return a0 + sub + (r % VT) * (kWide / VT / G) + (r / VT) * ngrp; };
   auto fetch = [&](int64_t a0) {
 #pragma unroll
     for (int r = 0; r < R; ++r) {
-      const int64_t a = a0 + sub + (int64_t)r * ngrp;
+      const int64_t a = row(a0, r);
       const int64_t ac = a < Nn ? a : Nn - 1;
       q0[r] = __ldg(S.node_ptr + ac);
       q1[r] = __ldg(S.node_ptr + ac + 1);
     }
   };
   fetch(grp - sub);
-  for (int64_t a0 = grp - sub; a0 < Nn; a0 += (int64_t)R * ngrp) {
+  for (int64_t a0 = grp - sub; a0 < Nn; a0 += (R / VT) * ngrp) {
     int64_t an[R], ac[R];
     int32_t p0[R], nb[R];
 #pragma unroll
     for (int r = 0; r < R; ++r) {
-      an[r] = a0 + sub + (int64_t)r * ngrp;
+      an[r] = row(a0, r);
       ac[r] = an[r] < Nn ? an[r] : Nn - 1;
       p0[r] = q0[r];
       nb[r] = q1[r] - q0[r];
     }
-    fetch(a0 + (int64_t)R * ngrp);
+    fetch(a0 + (R / VT) * ngrp);
     uint8_t kn[R];
 #pragma unroll
     for (int r = 0; r < R; ++r) kn[r] = S.known[ac[r] * D + lane % D];
@@ -517,14 +535,15 @@ __device__ __noinline__ double direction_apply(const SysT<T>& S, const T* z, con
         if (kn[r]) av = 0;
         pb[dof] = self[r];
         Ap[dof] = av;
-        pap.add_prod(self[r], av);
+        pap[r % VT].add_prod(self[r], av);
       }
     }
   }
-  return pap.value();
+#pragma unroll
+  for (int q = 0; q < VT; ++q) out[q][0] = pap[q].value();
 }
 
-template <int D, int G, typename T>
+template <int D, int G, typename T, int VT>
 __device__ void solve_instance(Ctx& c, const gfea_batch_instance& I, double delta2) {
   const int64_t Nn = I.n_nodes;
   BatchBuf<T> w;
@@ -533,17 +552,19 @@ __device__ void solve_instance(Ctx& c, const gfea_batch_instance& I, double delt
   const SysT<T> S{Nn, I.node_ptr, I.nbr, vals, I.known, I.translation_invariant};
   const SysT<double> S64{Nn, I.node_ptr, I.nbr, I.vals64, I.known, 0};
   const int tid = threadIdx.x;
-  const int64_t gtid = (int64_t)c.rank * blockDim.x + tid;
-  const int64_t nthr = (int64_t)kCL * blockDim.x;
+  // this thread's first virtual thread, and its real index (loops without sums)
+  const int64_t gtid = (int64_t)c.rank * kWide + tid;
+  const int64_t nthr = (int64_t)kCL * kWide;
+  const int64_t rtid = (int64_t)c.rank * (kWide / VT) + tid;
+  const int64_t rthr = (int64_t)kCL * (kWide / VT);
   const int lane = tid % G;
   const int64_t grp = gtid / G, ngrp = nthr / G;
-  const int64_t sub = grp % (32 / G);
   const double eps64 = 2.220446049250313e-16;
   const bool two_level = I.coarse.n_agg > 0;
 
   // block-Jacobi inverses (thread per node)
   double bad = 0;
-  for (int64_t a = gtid; a < Nn; a += nthr) {
+  for (int64_t a = rtid; a < Nn; a += rthr) {
     const int32_t p0 = S.node_ptr[a], p1 = S.node_ptr[a + 1];
     int lo = p0, hi = p1;
     while (lo < hi) {
@@ -576,9 +597,10 @@ __device__ void solve_instance(Ctx& c, const gfea_batch_instance& I, double delt
   }
 
   // FP64 residual of the start
-  double v4[4] = {0, 0, 0, bad}, o4[4];
-  resid64<D, G>(S64, I.b, I.x, w.r64, grp, ngrp, lane, v4);
-  csum<4>(c, v4, o4);
+  double v4[VT][4] = {}, o4[4];
+  v4[0][3] = bad;
+  resid64<D, G, VT>(S64, I.b, I.x, w.r64, grp, ngrp, lane, v4);
+  csum<4, VT>(c, v4, o4);
   double rr_true = o4[0];
   const double bb = o4[1];
   double floor2 = (32 * eps64) * (32 * eps64) * o4[2];
@@ -592,7 +614,7 @@ __device__ void solve_instance(Ctx& c, const gfea_batch_instance& I, double delt
     status = GFEA_ERR_NAN;
     finished = true;
   } else if (bb == 0) {  // b_i - A_ic x_c = 0: the unknowns are zero
-    for (int64_t a = gtid; a < Nn; a += nthr)
+    for (int64_t a = rtid; a < Nn; a += rthr)
 #pragma unroll
       for (int i = 0; i < D; ++i)
         if (!I.known[a * D + i]) I.x[a * D + i] = 0.0;
@@ -605,18 +627,18 @@ __device__ void solve_instance(Ctx& c, const gfea_batch_instance& I, double delt
 
   if (!finished) {
     // start: r = r64, dx = 0, p = 0, z = D^-1 r
-    for (int64_t a = gtid; a < Nn; a += nthr)
+    for (int64_t a = rtid; a < Nn; a += rthr)
 #pragma unroll
       for (int i = 0; i < D; ++i) {
         w.dx[a * D + i] = 0;
         w.pa[a * D + i] = 0;
       }
-    double v2[2] = {0, 0}, o2[2];
+    double v2[VT][2] = {}, o2[2];
     if (two_level)
-      restart_rz_two_level<D, T>(c, I, w, gtid, nthr, v2);
+      restart_rz_two_level<D, T, VT>(c, I, w, gtid, nthr, v2);
     else
-      restart_rz<D, T>(I, w, gtid, nthr, v2);
-    csum<2>(c, v2, o2);
+      restart_rz<D, T, VT>(I, w, gtid, nthr, v2);
+    csum<2, VT>(c, v2, o2);
     double rz = o2[0];
     double beta = 0;
     double trigger = fmax(delta2 * rr_true, 0.25 * tol2);
@@ -626,10 +648,12 @@ __device__ void solve_instance(Ctx& c, const gfea_batch_instance& I, double delt
     T* pb = w.pb;
     const bool diff = sizeof(T) == 4 && S.diff;
     for (;;) {
-      double va[1], oa[1];
-      va[0] = diff ? direction_apply<D, G, T, true>(S, w.z, pa, pb, w.Ap, (T)beta, grp, ngrp, lane)
-                   : direction_apply<D, G, T, false>(S, w.z, pa, pb, w.Ap, (T)beta, grp, ngrp, lane);
-      csum<1>(c, va, oa);
+      double va[VT][1], oa[1];
+      if (diff)
+        direction_apply<D, G, T, true, VT>(S, w.z, pa, pb, w.Ap, (T)beta, grp, ngrp, lane, va);
+      else
+        direction_apply<D, G, T, false, VT>(S, w.z, pa, pb, w.Ap, (T)beta, grp, ngrp, lane, va);
+      csum<1, VT>(c, va, oa);
       const double pap = oa[0];
       if (!(pap > 0) || !isfinite(pap)) {
         status = isfinite(pap) ? GFEA_ERR_BREAKDOWN : GFEA_ERR_NAN;
@@ -637,17 +661,16 @@ __device__ void solve_instance(Ctx& c, const gfea_batch_instance& I, double delt
       }
       const double alpha = rz / pap;
       // x, r, z update; partials r.z, r.r
-      double vb[2] = {0, 0}, ob[2];
-      DotAcc<T> rz_acc, rr_acc;
+      double vb[VT][2], ob[2];
       const T al = (T)alpha;
       if (two_level) {  // x, r; then the coarse correction; then z
         constexpr int B = 4;  // unknowns per thread with their loads in flight
         const int64_t N = Nn * D;
-        for (int64_t d0 = gtid; d0 < N; d0 += B * nthr) {
+        for (int64_t d0 = rtid; d0 < N; d0 += B * rthr) {
           T xo[B], po[B], ro[B], ao[B];
 #pragma unroll
           for (int q = 0; q < B; ++q) {
-            const int64_t dof = d0 + q * nthr < N ? d0 + q * nthr : d0;
+            const int64_t dof = d0 + q * rthr < N ? d0 + q * rthr : d0;
             xo[q] = ldcg(w.dx + dof);
             po[q] = ldcg(pb + dof);
             ro[q] = ldcg(w.r + dof);
@@ -655,39 +678,44 @@ __device__ void solve_instance(Ctx& c, const gfea_batch_instance& I, double delt
           }
 #pragma unroll
           for (int q = 0; q < B; ++q) {
-            const int64_t dof = d0 + q * nthr;
+            const int64_t dof = d0 + q * rthr;
             if (dof < N) {
               w.dx[dof] = xo[q] + al * po[q];
               w.r[dof] = ro[q] - al * ao[q];
             }
           }
         }
-        coarse_correct<D, T>(c, I, w.r, gtid, nthr);
-        z_two_level<D, T>(I, w, gtid, nthr, rz_acc, rr_acc);
-      } else
-      for (int64_t a = gtid; a < Nn; a += nthr) {
-        T rl[D];
+        coarse_correct<D, T>(c, I, w.r, rtid, rthr);
+        z_two_level<D, T, VT>(I, w, gtid, nthr, vb);
+      } else {
 #pragma unroll
-        for (int i = 0; i < D; ++i) {
-          const int64_t dof = a * D + i;
-          w.dx[dof] = ldcg(w.dx + dof) + al * ldcg(pb + dof);
-          rl[i] = ldcg(w.r + dof) - al * ldcg(w.Ap + dof);
-          w.r[dof] = rl[i];
-        }
+        for (int q = 0; q < VT; ++q) {
+          DotAcc<T> rz_acc, rr_acc;
+          for (int64_t a = gtid + q * (kWide / VT); a < Nn; a += nthr) {
+            T rl[D];
 #pragma unroll
-        for (int i = 0; i < D; ++i) {
-          T zi = 0;
+            for (int i = 0; i < D; ++i) {
+              const int64_t dof = a * D + i;
+              w.dx[dof] = ldcg(w.dx + dof) + al * ldcg(pb + dof);
+              rl[i] = ldcg(w.r + dof) - al * ldcg(w.Ap + dof);
+              w.r[dof] = rl[i];
+            }
 #pragma unroll
-          for (int j = 0; j < D; ++j) zi += w.dinv[a * D * D + i * D + j] * rl[j];
-          if (I.known[a * D + i]) zi = 0;
-          w.z[a * D + i] = zi;
-          rz_acc.add_prod(rl[i], zi);
-          rr_acc.add_prod(rl[i], rl[i]);
+            for (int i = 0; i < D; ++i) {
+              T zi = 0;
+#pragma unroll
+              for (int j = 0; j < D; ++j) zi += ldcg(w.dinv + a * D * D + i * D + j) * rl[j];
+              if (I.known[a * D + i]) zi = 0;
+              w.z[a * D + i] = zi;
+              rz_acc.add_prod(rl[i], zi);
+              rr_acc.add_prod(rl[i], rl[i]);
+            }
+          }
+          vb[q][0] = rz_acc.value();
+          vb[q][1] = rr_acc.value();
         }
       }
-      vb[0] = rz_acc.value();
-      vb[1] = rr_acc.value();
-      csum<2>(c, vb, ob);
+      csum<2, VT>(c, vb, ob);
       beta = ob[0] / rz;
       rz = ob[0];
       const double rr_it = ob[1];
@@ -701,7 +729,7 @@ __device__ void solve_instance(Ctx& c, const gfea_batch_instance& I, double delt
       }
       if (rr_it > trigger && iters < I.max_iters) continue;
       // reliable update: x += dx in FP64, then the FP64 residual replaces r
-      for (int64_t a = gtid; a < Nn; a += nthr)
+      for (int64_t a = rtid; a < Nn; a += rthr)
 #pragma unroll
         for (int i = 0; i < D; ++i) {
           const int64_t dof = a * D + i;
@@ -709,9 +737,9 @@ __device__ void solve_instance(Ctx& c, const gfea_batch_instance& I, double delt
           w.dx[dof] = 0;
         }
       c.cl.sync();  // the updated x of every node is visible before the residual reads neighbours
-      double vr[4] = {0, 0, 0, 0}, orr[4];
-      resid64<D, G>(S64, I.b, I.x, w.r64, grp, ngrp, lane, vr);
-      csum<4>(c, vr, orr);
+      double vr[VT][4] = {}, orr[4];
+      resid64<D, G, VT>(S64, I.b, I.x, w.r64, grp, ngrp, lane, vr);
+      csum<4, VT>(c, vr, orr);
       rr_true = orr[0];
       ++updates;
       floor2 = (32 * eps64) * (32 * eps64) * orr[2];
@@ -728,12 +756,12 @@ __device__ void solve_instance(Ctx& c, const gfea_batch_instance& I, double delt
       stall = rr_true > 0.9 * rr_best ? stall + 1 : 0;
       rr_best = fmin(rr_best, rr_true);
       if (stall >= 8) break;
-      double vz[2] = {0, 0}, oz[2];
+      double vz[VT][2] = {}, oz[2];
       if (two_level)
-        restart_rz_two_level<D, T>(c, I, w, gtid, nthr, vz);
+        restart_rz_two_level<D, T, VT>(c, I, w, gtid, nthr, vz);
       else
-        restart_rz<D, T>(I, w, gtid, nthr, vz);
-      csum<2>(c, vz, oz);
+        restart_rz<D, T, VT>(I, w, gtid, nthr, vz);
+      csum<2, VT>(c, vz, oz);
       beta = next_beta(2, oz[0], rz, beta);
       rz = oz[0];
       trigger = fmax(delta2 * rr_true, 0.25 * tol2);
@@ -750,12 +778,12 @@ __device__ void solve_instance(Ctx& c, const gfea_batch_instance& I, double delt
   }
 }
 
-template <typename T>
+template <typename T, int VT>
 __device__ void dispatch(Ctx& c, const gfea_batch_instance& I, double delta2) {
   switch (I.dof_n) {
-    case 1: solve_instance<1, 8, T>(c, I, delta2); break;
-    case 2: solve_instance<2, 8, T>(c, I, delta2); break;
-    default: solve_instance<3, 32, T>(c, I, delta2); break;
+    case 1: solve_instance<1, 8, T, VT>(c, I, delta2); break;
+    case 2: solve_instance<2, 8, T, VT>(c, I, delta2); break;
+    default: solve_instance<3, 32, T, VT>(c, I, delta2); break;
   }
 }
 
@@ -772,11 +800,22 @@ __global__ void __cluster_dims__(kCL, 1, 1) __launch_bounds__(BT, 2 * kNarrow / 
   if (BT == kWide) cudaTriggerProgrammaticLaunchCompletion();
   Ctx c{cg::this_cluster(), 0, slots, sh, 0};
   c.rank = c.cl.block_rank();
-  int split = 0, hi = n;  // the wide systems are [0, split)
-  while (split < hi) {
-    const int mid = (split + hi) >> 1;
-    if (stored_values(insts[mid]) >= kWideValues) split = mid + 1; else hi = mid;
+  // the wide systems are [0, split): none where the batch fills the narrow
+  // clusters for longer than its largest system takes
+  int split = 0;
+  double total = 0;
+  for (int i = threadIdx.x; i < n; i += BT) total += (double)stored_values(insts[i]);
+  total = block_sum(total, sh);
+  if (threadIdx.x == 0) s_idx = (double)stored_values(insts[0]) * (2 * kSMs / kCL) > 2 * total;
+  __syncthreads();
+  if (s_idx) {
+    int hi = n;
+    while (split < hi) {
+      const int mid = (split + hi) >> 1;
+      if (stored_values(insts[mid]) >= kWideValues) split = mid + 1; else hi = mid;
+    }
   }
+  __syncthreads();
   const int first = BT == kWide ? 0 : split, last = BT == kWide ? split : n;
   for (;;) {
     if (c.rank == 0 && threadIdx.x == 0) s_idx = first + atomicAdd(next + (BT == kWide ? 0 : 1), 1);
@@ -785,7 +824,7 @@ __global__ void __cluster_dims__(kCL, 1, 1) __launch_bounds__(BT, 2 * kNarrow / 
     c.cl.sync();  // rank 0's slot is read by all before it changes
     if (idx >= last) break;
     const gfea_batch_instance I = insts[idx];
-    dispatch<T>(c, I, delta2);
+    dispatch<T, kWide / BT>(c, I, delta2);
   }
   if (BT == kNarrow) cudaGridDependencySynchronize();
 }

@@ -1,6 +1,6 @@
 """Batched PCG with systems on both sides of the wide-cluster limit (400 000
 stored values): solutions against single FP64 solves, and bit-equality alone
-and in company."""
+(wide) and in company (wide, or narrow in a batch that fills the GPU)."""
 
 import numpy as np
 import pytest
@@ -46,3 +46,17 @@ def test_widths(precision, names):
         s.x.copy_(x)
         solve_batch([s], precision=precision, coarse=0)
         assert np.array_equal(s.x.cpu().numpy(), m)
+
+
+@pytest.mark.parametrize("name", ["wide2d", "wide3d"])
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+def test_same_bits_at_either_width(precision, name):
+    from easyfea_gb300.batching import solve_batch
+
+    systems = [elastic_system(MESHES[name](), 210000.0)[1] for _ in range(24)]  # 38 largest > 2 x 24: no
+    x0 = systems[0].x.clone()
+    solve_batch(systems, precision=precision, coarse=0)
+    narrow = systems[0].x.cpu().numpy()  # (each system's K has its own rounding: atomics)
+    systems[0].x.copy_(x0)
+    solve_batch(systems[:1], precision=precision, coarse=0)
+    assert np.array_equal(systems[0].x.cpu().numpy(), narrow)
