@@ -842,6 +842,7 @@ int launch_widths(const gfea_batch_instance* desc, int n, int* next, double delt
   GFEA_CUDA_TRY(cudaOccupancyMaxActiveClusters(&resident, batch_pcg_kernel<T, kWide>, &cfg));
   cfg.gridDim = dim3(kCL * std::max(1, std::min(n, resident)));
   GFEA_CUDA_TRY(cudaLaunchKernelEx(&cfg, batch_pcg_kernel<T, kWide>, desc, n, next, delta2));
+  GFEA_LAUNCH_CHECK();
   cudaLaunchAttribute overlap = {};
   overlap.id = cudaLaunchAttributeProgrammaticStreamSerialization;
   overlap.val.programmaticStreamSerializationAllowed = 1;
@@ -850,6 +851,7 @@ int launch_widths(const gfea_batch_instance* desc, int n, int* next, double delt
   cfg.blockDim = dim3(kNarrow);
   cfg.gridDim = dim3(kCL * std::max(1, std::min(n, 2 * kSMs / kCL)));
   GFEA_CUDA_TRY(cudaLaunchKernelEx(&cfg, batch_pcg_kernel<T, kNarrow>, desc, n, next, delta2));
+  GFEA_LAUNCH_CHECK();
   return GFEA_OK;
 }
 
