@@ -41,6 +41,15 @@ namespace gfea {
 
 constexpr int kSMs = 152;  // GB300 streaming multiprocessors (two dies x 76)
 
+// Shared memory above 48 KB (static part included) is an attribute of a kernel
+// on one device, so every launch asks for it on the current one (a host call,
+// < 1 us).  'most' is the kernel's largest dynamic part, not the launch's:
+// another thread may be launching it with more.
+template <typename K>
+cudaError_t allow_smem(K* kern, size_t most) {
+  return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most);
+}
+
 __host__ __device__ inline int64_t ceil_div(int64_t a, int64_t b) { return (a + b - 1) / b; }
 
 // ---------------------------------------------------------------------------

@@ -23,7 +23,6 @@
 #include <math.h>
 
 #include <algorithm>
-#include <mutex>
 
 #include "common.cuh"
 #include "ff.cuh"
@@ -304,13 +303,7 @@ int coarse_inverse(const CoarseDev& C, double zero_tol, double shift, cudaStream
     if (grid == 0) return GFEA_ERR_ARG;
   }
   const size_t smem = tile_smem(best);
-  static std::once_flag once;
-  static cudaError_t attr = cudaSuccess;
-  std::call_once(once, [&] {
-    attr = cudaFuncSetAttribute(coarse_inverse_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                (int)tile_smem(Tile{kTileMax, kTileMax, 1}));
-  });
-  GFEA_CUDA_TRY(attr);
+  GFEA_CUDA_TRY(allow_smem(coarse_inverse_kernel, tile_smem(Tile{kTileMax, kTileMax, 1})));
   uint32_t* bar = reinterpret_cast<uint32_t*>(C.pinvh);
   GFEA_CUDA_TRY(cudaMemsetAsync(bar, 0, sizeof(uint32_t), st));
   cudaLaunchConfig_t cfg{};

@@ -46,7 +46,6 @@
 #include <stdlib.h>
 
 #include <algorithm>
-#include <mutex>
 
 #include "coarse.cuh"
 #include "common.cuh"
@@ -1018,10 +1017,7 @@ __global__ void __launch_bounds__(kRT, 1) resident_kernel(ResidentProblem<T> P, 
 template <int D, int G, typename T>
 int launch(const ResidentProblem<T>& P, const ResidentGeom& g, cudaStream_t st) {
   auto kern = resident_kernel<D, G, T>;
-  static std::once_flag once;
-  static cudaError_t attr = cudaSuccess;
-  std::call_once(once, [&] { attr = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kRSmemMax); });
-  GFEA_CUDA_TRY(attr);
+  GFEA_CUDA_TRY(allow_smem(kern, kRSmemMax));
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = dim3(g.grid);
   cfg.blockDim = dim3(kRT);

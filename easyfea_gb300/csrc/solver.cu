@@ -1538,10 +1538,7 @@ int launch_apply_staged(const SysT<T>& S, const StageGeom& g, const unsigned cha
                         double* partials, Scal* sc, cudaStream_t st) {
   auto kern = apply_staged_kernel<D, T, DIFF>;
   const size_t smem = (size_t)g.stages * g.tile_bytes;
-  static std::once_flag once;
-  static cudaError_t attr = cudaSuccess;
-  std::call_once(once, [&] { attr = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemMax); });
-  GFEA_CUDA_TRY(attr);
+  GFEA_CUDA_TRY(allow_smem(kern, kSmemMax));
   static std::atomic<int64_t> occ{0};  // (smem << 8) | blocks per SM of the last query
   int64_t o = occ.load(std::memory_order_relaxed);
   int per_sm = (int)(o & 255);

@@ -1,0 +1,65 @@
+"""Which kernels a solve launches, and with what grids and shared memory, on
+devices this machine does not have: a fake CUDA runtime records the launches of
+the built library and refuses what the real one would refuse."""
+
+import json
+import os
+import subprocess
+import sys
+
+import pytest
+
+from easyfea_gb300 import _build
+
+HERE = os.path.dirname(os.path.abspath(__file__))
+
+
+@pytest.fixture(scope="module")
+def run(tmp_path_factory):
+    _build.build()
+    d = tmp_path_factory.mktemp("fake")
+    script = d / "fake.map"
+    script.write_text("libcudart.so.13 { global: *; };\n")
+    so = str(d / "libcudart.so.13")
+    inc = os.path.join(os.path.dirname(os.path.dirname(os.path.realpath(_build.nvcc_path()))), "include")
+    r = subprocess.run(["g++", "-shared", "-fPIC", "-O1", "-std=c++17", "-I", inc, "-Wl,-soname,libcudart.so.13",
+                        f"-Wl,--version-script={script}", "-o", so, os.path.join(HERE, "fake_cudart.cpp")],
+                       capture_output=True, text=True)
+    assert r.returncode == 0, r.stderr
+
+    def go(*steps, env=None):
+        r = subprocess.run([sys.executable, os.path.join(HERE, "host_dispatch.py"), so, json.dumps(steps)],
+                           capture_output=True, text=True, timeout=120, env={**os.environ, **(env or {})})
+        assert r.returncode == 0, r.stderr[-2000:]
+        return json.loads(r.stdout.strip().splitlines()[-1])
+
+    return go
+
+
+def names(step):
+    return [line.split()[0] for line in step["launches"]]
+
+
+def refused(step):
+    return [line for line in step["launches"] if line.endswith("refused")]
+
+
+BOX = {"D": 3, "nodes": 13104, "degree": 24, "precision": "fp64"}
+
+
+@pytest.mark.parametrize("case,kernel", [
+    ({**BOX}, "resident_kernel"),
+    ({**BOX, "precision": "mixed"}, "resident_kernel"),
+    ({"D": 2, "nodes": 2106, "degree": 7, "precision": "mixed"}, "resident_kernel"),  # 40 to 48 KB
+    ({**BOX, "nodes": 100000, "coarse": 250}, "coarse_inverse"),
+    ({**BOX, "precision": "mixed", "coarse": 0, "check_every": 4, "env": {"GFEA_STAGE_MIN_BYTES": "0"}},
+     "apply_staged_kernel"),
+])
+def test_shared_memory_is_opted_into_on_every_device(run, case, kernel):
+    """The attribute belongs to the device that was current when it was set: a
+    second device of the same process has to get it too."""
+    out = run({**case, "device": 0}, {**case, "device": 1})
+    for s in out:
+        assert any(n.startswith(kernel) for n in names(s)), names(s)
+        assert not refused(s)
+    assert names(out[0]) == names(out[1])
