@@ -12,14 +12,16 @@
 // So a step is one barrier, the pivot block's inverse (by every CTA), P B_KJ
 // for the tile's columns and the rank-16 update of the tile.
 //
+// The trailing updates run on pairs; P and P B_KJ are FP64, as in the two
+// launches per pivot block this replaces (pairs there lost up to two decades
+// against an inverse in extended precision where aggregates have one or two
+// nodes: 384 unknowns of HEXA8, relative error 2.2e-2 instead of 8e-5).
+//
 // Bound: latency -- per step a barrier (~2 us), the panel's trip through L2,
 // the 16 dependent pivots -- and for n > 1000 the FP32 pipe (13 operations a
-// product).  The two launches per pivot block it replaces took ~40 us a pair,
-// most of it FP64 divisions and conversions of the pivot block's inverse,
-// which every block repeated on the FP64 pipe.  Before -> now: n = 33 0.10 ->
-// 0.05 ms, 192 0.45 -> 0.12, 429 1.26 -> 0.36, 612 1.80 -> 0.60, 1152 3.76 ->
-// 2.04; the error against extended precision is the same (median ratio 0.94
-// over 72 random matrices of 33 to 300 unknowns).
+// product).  The two launches took ~40 us a pair, most of it the pivot block's
+// inverse, which every block repeated on the FP64 pipe.  Before -> now:
+// n = 33 0.10 -> 0.06 ms, 192 0.45 -> 0.13, 612 1.80 -> 0.75, 1152 3.76 -> 2.50.
 #include <math.h>
 
 #include <algorithm>
@@ -35,6 +37,7 @@ namespace {
 constexpr int kB = 16;        // pivot block
 constexpr int kIT = 256;      // threads per CTA
 constexpr int kTileMax = 128; // rows and columns of a tile
+constexpr double kIllResidual = 1e-8;  // of a pivot block inverted in pairs
 
 struct Tile {
   int rows, cols;  // tile size (multiples of kB)
@@ -44,6 +47,7 @@ struct Tile {
 // Shared memory: tile (hi, lo), raw rows for the tile's columns and rows,
 // pivot block (two states), P B_KJ.
 __host__ __device__ inline size_t tile_smem(const Tile& t) {
+  static_assert(sizeof(float2) == sizeof(double), "a pair and a double take the same room");
   return sizeof(float2) * ((size_t)t.rows * t.cols + (size_t)kB * (t.cols + t.rows) + 2 * kB * (kB + 1) +
                            (size_t)kB * t.cols);
 }
@@ -86,8 +90,8 @@ __global__ void __launch_bounds__(kIT, 1) coarse_inverse_kernel(double* __restri
   __shared__ int s_ok;
   __shared__ double D[2][kB][kB + 1];
   float2* B = reinterpret_cast<float2*>(smem);              // rows x cols
-  float2* RJ = B + T.rows * T.cols;                         // kB x cols: raw rows at the tile's columns
-  float2* RI = RJ + kB * T.cols;                            // rows x kB: at the tile's rows (transposed, signed)
+  double* RJ = reinterpret_cast<double*>(B + T.rows * T.cols);  // kB x cols: raw rows at the tile's columns
+  float2* RI = reinterpret_cast<float2*>(RJ + kB * T.cols);     // rows x kB: at the tile's rows (transposed, signed)
   float2(*M)[kB][kB + 1] = reinterpret_cast<float2(*)[kB][kB + 1]>(RI + kB * T.rows);
   float2* PR = RI + kB * T.rows + 2 * kB * (kB + 1);        // kB x cols
   const int tid = threadIdx.x, lane = tid & 31;
@@ -148,7 +152,10 @@ __global__ void __launch_bounds__(kIT, 1) coarse_inverse_kernel(double* __restri
       const int l = tid / kB, c = tid % kB;
       M[0][l][c] = raw(l, k0 + c);
     }
-    for (int e = tid; e < kB * T.cols; e += kIT) RJ[e] = raw(e / T.cols, j0 + e % T.cols);
+    for (int e = tid; e < kB * T.cols; e += kIT) {
+      const float2 v = raw(e / T.cols, j0 + e % T.cols);
+      RJ[e] = (double)v.x + (double)v.y;
+    }
     for (int e = tid; e < kB * T.rows; e += kIT) {
       const int l = e / T.rows, i = i0 + e % T.rows;
       float2 v = raw(l, i);
@@ -176,11 +183,12 @@ __global__ void __launch_bounds__(kIT, 1) coarse_inverse_kernel(double* __restri
     }
     static_assert(kB % 2 == 0 && kIT == kB * kB, "P ends in M[0], one element per thread");
     // the pairs lose the block's condition number; one step
-    // P <- P + P (I - B_KK P) with the residual in FP64 (its product with P
-    // needs few digits) restores it.  A block too ill-conditioned for that
-    // (rotations of one- or two-node aggregates leave pivots at the level of
-    // the shift) is inverted and multiplied in FP64, ~15 us slower.
-    bool ill;
+    // P <- P + P (I - B_KK P) with the residual in FP64 restores it to FP64
+    // (its product with P needs few digits while the residual is below 1e-8,
+    // whose square and whose 2^-24 are lost on P).  A block too
+    // ill-conditioned for that (rotations of one- or two-node aggregates leave
+    // pivots at the level of the shift) is inverted in FP64, ~15 us slower.
+    // P stays in FP64 for P B_KJ.
     {
       const int i = tid / kB, j = tid % kB;
       const float2 b = raw(i, k0 + j), p0 = M[0][i][j];
@@ -192,13 +200,11 @@ __global__ void __launch_bounds__(kIT, 1) coarse_inverse_kernel(double* __restri
 #pragma unroll
       for (int q = 0; q < kB; ++q) e -= D[0][i][q] * D[1][q][j];
       M[1][i][j].x = (float)e;
-      ill = __syncthreads_or(!(fabs(e) <= 1e-6));
-      if (!ill) {
+      if (!__syncthreads_or(!(fabs(e) <= kIllResidual))) {
         float c = 0.f;
 #pragma unroll
         for (int q = 0; q < kB; ++q) c += M[0][i][q].x * M[1][q][j].x;
-        __syncthreads();
-        ff_split(p64 + (double)c, M[0][i][j].x, M[0][i][j].y);
+        D[0][i][j] = p64 + (double)c;
       } else {
 #pragma unroll 1
         for (int p = 0; p < kB; ++p) {
@@ -208,28 +214,21 @@ __global__ void __launch_bounds__(kIT, 1) coarse_inverse_kernel(double* __restri
           D[(p + 1) & 1][i][j] = i == p ? pj : (j == p ? 0.0 : S[i][j]) - S[i][p] * pj;
           __syncthreads();
         }
-        ff_split(D[0][i][j], M[0][i][j].x, M[0][i][j].y);
       }
       __syncthreads();
     }
-    const float2(*P)[kB + 1] = M[0];
+    const double(*P)[kB + 1] = D[0];
     // P B_KJ (columns of the pivot block itself: P)
     for (int e = tid; e < kB * T.cols; e += kIT) {
       const int l = e / T.cols, c = e % T.cols, j = j0 + c;
-      float2 s = make_float2(0.f, 0.f);
+      double t = 0;
       if (j >= k0 && j < k0 + kB) {
-        s = P[l][j - k0];
-      } else if (ill) {
-        double t = 0;
-#pragma unroll
-        for (int q = 0; q < kB; ++q)
-          t += D[0][l][q] * ((double)RJ[q * T.cols + c].x + (double)RJ[q * T.cols + c].y);
-        ff_split(t, s.x, s.y);
+        t = P[l][j - k0];
       } else {
 #pragma unroll
-        for (int q = 0; q < kB; ++q) ff_fma_acc(s.x, s.y, P[l][q].x, P[l][q].y, RJ[q * T.cols + c].x, RJ[q * T.cols + c].y);
+        for (int q = 0; q < kB; ++q) t += P[l][q] * RJ[q * T.cols + c];
       }
-      PR[e] = s;
+      ff_split(t, PR[e].x, PR[e].y);
     }
     __syncthreads();
     // the tile: a thread owns one column for a share of the rows
