@@ -13,6 +13,12 @@ __device__ __forceinline__ void ff_split(double d, float& hi, float& lo) {
   lo = (float)(d - (double)hi);
 }
 
+__device__ __forceinline__ float2 ff_pair(double d) {
+  float2 v;
+  ff_split(d, v.x, v.y);
+  return v;
+}
+
 // (sh, sl) += (ah, al) (bh, bl); the al bl term is below the pair's precision
 __device__ __forceinline__ void ff_fma_acc(float& sh, float& sl, float ah, float al, float bh, float bl) {
   const float p = ah * bh;

@@ -1,27 +1,30 @@
-// Inverse of the two-level preconditioner's SPD coarse matrix in one
-// cooperative launch.
+// Inverse of the two-level preconditioner's SPD coarse matrix, a launch per
+// pivot block.
 //
 // In-place blocked Gauss-Jordan (no pivoting: every pivot block of an SPD
 // matrix is SPD) on float-float pairs.  For the pivot block K of B =
 // [[B_KK, B_KJ], [B_IK, B_IJ]], with P = B_KK^-1:
 //   B_KK <- P,  B_KJ <- P B_KJ,  B_IK <- -B_IK P,  B_IJ <- B_IJ - B_IK P B_KJ.
-// Every CTA keeps one tile of B in shared memory for the whole inversion.  A
-// step reads only the raw rows B_K* (16 x n, published by the tiles that own
-// them at the end of the step before): the columns B_*K are the same numbers,
-// B_iK = B_Ki^T for rows not yet eliminated and -B_Ki^T for those that are.
-// So a step is one barrier, the pivot block's inverse (by every CTA), P B_KJ
-// for the tile's columns and the rank-16 update of the tile.
+// A CTA owns one tile of B.  A step reads only the raw rows B_K* (16 x n,
+// published by the tiles that own them at the end of the step before): the
+// columns B_*K are the same numbers, B_iK = B_Ki^T for rows not yet eliminated
+// and -B_Ki^T for those that are.  So a step is one launch: the pivot block's
+// inverse (by every CTA), P B_KJ for the tile's columns and the rank-16 update
+// of the tile.  Nothing waits on another CTA: any number of SMs does, and no
+// wait can run out.  Each launch is a programmatic dependent of the one before,
+// which hides part of the gap between them.
 //
-// The trailing updates run on pairs; P and P B_KJ are FP64, as in the two
-// launches per pivot block this replaces (pairs there lost up to two decades
-// against an inverse in extended precision where aggregates have one or two
-// nodes: 384 unknowns of HEXA8, relative error 2.2e-2 instead of 8e-5).
+// The trailing updates run on pairs; P and P B_KJ are FP64 (pairs there lost up
+// to two decades against an inverse in extended precision where aggregates
+// have one or two nodes: 384 unknowns of HEXA8, relative error 2.2e-2 instead
+// of 8e-5).
 //
-// Bound: latency -- per step a barrier (~2 us), the panel's trip through L2,
-// the 16 dependent pivots -- and for n > 1000 the FP32 pipe (13 operations a
-// product).  The two launches took ~40 us a pair, most of it the pivot block's
-// inverse, which every block repeated on the FP64 pipe.  Before -> now:
-// n = 33 0.10 -> 0.06 ms, 192 0.45 -> 0.13, 612 1.80 -> 0.75, 1152 3.76 -> 2.50.
+// Bound: latency -- per step the launch (~2 us), the panel's and the tile's
+// trips through L2, the 16 dependent pivots -- and for n > 1000 the FP32 pipe
+// (13 operations a product).  Two launches per pivot block with the block's
+// inverse in FP64 by every block -> this (all steps in one cooperative launch
+// with the tiles kept in shared memory): n = 33 0.10 -> 0.06 ms (0.06), 192
+// 0.45 -> 0.15 (0.14), 612 1.80 -> 0.75 (0.62), 1152 3.76 -> 2.32 (1.79).
 #include <math.h>
 
 #include <algorithm>
@@ -29,14 +32,13 @@
 #include "common.cuh"
 #include "ff.cuh"
 #include "inverse.cuh"
-#include "stage.cuh"
 
 namespace gfea {
 namespace {
 
 constexpr int kB = 16;        // pivot block
 constexpr int kIT = 256;      // threads per CTA
-constexpr int kTileMax = 128; // rows and columns of a tile
+constexpr size_t kSmemMax = 216 * 1024;  // dynamic shared memory
 constexpr double kIllResidual = 1e-8;  // of a pivot block inverted in pairs
 
 struct Tile {
@@ -52,134 +54,123 @@ __host__ __device__ inline size_t tile_smem(const Tile& t) {
                            (size_t)kB * t.cols);
 }
 
-__device__ __forceinline__ uint32_t ld_acquire(const uint32_t* p) {
-  uint32_t v;
-  asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
-  return v;
-}
-
-// All CTAs have arrived (bounded wait); their earlier writes are visible
-// through ld.cg.
-__device__ bool grid_barrier(uint32_t* bar, uint32_t target, int* ok) {
-  if (gridDim.x == 1) {
-    __syncthreads();
-    return true;
-  }
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    __threadfence();
-    atomicAdd(bar, 1u);
-    const uint64_t t0 = global_ns();
-    bool good = true;
-    for (uint32_t i = 1; (int32_t)(ld_acquire(bar) - target) < 0; ++i)
-      if ((i & 255u) == 0 && global_ns() - t0 > kWaitLimitNs) {
-        good = false;
-        break;
-      }
-    *ok = good;
-  }
-  __syncthreads();
-  return *ok != 0;
-}
-
-__global__ void __launch_bounds__(kIT, 1) coarse_inverse_kernel(double* __restrict__ A, int n, Tile T, float* h0,
-                                                                float* l0, float* h1, float* l1, uint32_t* bar,
-                                                                double zero_tol, double shift) {
-  extern __shared__ __align__(16) unsigned char smem[];
+// The largest diagonal entry (non-negative doubles order like their bits).
+__device__ double largest_diagonal(const double* __restrict__ A, int n) {
   __shared__ unsigned long long s_max[kIT / 32];
-  __shared__ int s_ok;
-  __shared__ double D[2][kB][kB + 1];
-  float2* B = reinterpret_cast<float2*>(smem);              // rows x cols
-  double* RJ = reinterpret_cast<double*>(B + T.rows * T.cols);  // kB x cols: raw rows at the tile's columns
-  float2* RI = reinterpret_cast<float2*>(RJ + kB * T.cols);     // rows x kB: at the tile's rows (transposed, signed)
-  float2(*M)[kB][kB + 1] = reinterpret_cast<float2(*)[kB][kB + 1]>(RI + kB * T.rows);
-  float2* PR = RI + kB * T.rows + 2 * kB * (kB + 1);        // kB x cols
-  const int tid = threadIdx.x, lane = tid & 31;
-  const int i0 = (blockIdx.x / T.gc) * T.rows, j0 = (blockIdx.x % T.gc) * T.cols;
-  float *ph[2] = {h0, h1}, *pl[2] = {l0, l1};
-  if (tid == 0) s_ok = 1;
-
-  // largest diagonal entry: a unit diagonal for empty or fully constrained
-  // coarse unknowns, a relative shift elsewhere (rotations of degenerate
-  // aggregates)
-  unsigned long long m = 0;  // non-negative doubles order like their bits
-  for (int i = tid; i < n; i += kIT)
-    m = max(m, (unsigned long long)__double_as_longlong(fabs(__ldcg(A + (int64_t)i * n + i))));
+  unsigned long long m = 0;
+  for (int i = threadIdx.x; i < n; i += kIT)
+    m = max(m, (unsigned long long)__double_as_longlong(fabs(A[(int64_t)i * n + i])));
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) m = max(m, __shfl_xor_sync(0xffffffffu, m, o));
-  if (lane == 0) s_max[tid / 32] = m;
+  if (threadIdx.x % 32 == 0) s_max[threadIdx.x / 32] = m;
   __syncthreads();
 #pragma unroll
   for (int w = 0; w < kIT / 32; ++w) m = max(m, s_max[w]);
-  const double dmax = m > 0 ? __longlong_as_double((long long)m) : 1.0;
+  return m > 0 ? __longlong_as_double((long long)m) : 1.0;
+}
 
-  // the tile; beyond n the identity
+// Entry (i, j) of the regularised matrix, beyond n the identity: a unit
+// diagonal (the largest entry) for empty or fully constrained coarse unknowns,
+// a relative shift elsewhere (rotations of degenerate aggregates).
+__device__ __forceinline__ double regularised(const double* __restrict__ A, int n, int i, int j, double dmax,
+                                              double zero_tol, double shift) {
+  if (i >= n || j >= n) return i == j ? 1.0 : 0.0;
+  const double v = A[(int64_t)i * n + j];
+  return i != j ? v : (v > zero_tol * dmax ? v + shift * dmax : dmax);
+}
+
+// Ahead of the steps: the largest diagonal entry and the raw rows of the first
+// pivot block.
+__global__ void __launch_bounds__(kIT) coarse_inverse_start_kernel(const double* __restrict__ A, int n,
+                                                                   float2* rows, double* scale, double zero_tol,
+                                                                   double shift) {
+  const double dmax = largest_diagonal(A, n);
+  if (blockIdx.x == 0 && threadIdx.x == 0) *scale = dmax;
+  const int j = blockIdx.x * kIT + threadIdx.x;
+  if (j < n)
+#pragma unroll
+    for (int l = 0; l < kB; ++l)
+      if (l < n) rows[(int64_t)l * n + j] = ff_pair(regularised(A, n, l, j, dmax, zero_tol, shift));
+}
+
+// Steps [first, last) of the inversion.  Between two launches A holds the
+// tile's pairs in the place of its doubles.
+__global__ void __launch_bounds__(kIT) coarse_inverse_kernel(double* A, int n, Tile T, float2* rows0,
+                                                             float2* rows1, const double* scale, int first, int last,
+                                                             double zero_tol, double shift) {
+  extern __shared__ __align__(16) unsigned char smem[];
+  __shared__ double D[2][kB][kB + 1];
+  float2* B = reinterpret_cast<float2*>(smem);                  // rows x cols
+  double* RJ = reinterpret_cast<double*>(B + T.rows * T.cols);  // kB x cols: raw rows at the tile's columns
+  float2* RI = reinterpret_cast<float2*>(RJ + kB * T.cols);     // rows x kB: at the tile's rows (transposed, signed)
+  float2(*M)[kB][kB + 1] = reinterpret_cast<float2(*)[kB][kB + 1]>(RI + kB * T.rows);
+  float2* PR = RI + kB * T.rows + 2 * kB * (kB + 1);            // kB x cols
+  float2* A2 = reinterpret_cast<float2*>(A);
+  cudaGridDependencySynchronize();            // the step before is complete
+  cudaTriggerProgrammaticLaunchCompletion();  // the next one may take its place on the SMs
+  const int tid = threadIdx.x;
+  const int i0 = (int)(blockIdx.x / T.gc) * T.rows, j0 = (int)(blockIdx.x % T.gc) * T.cols;
+  float2* rows[2] = {rows0, rows1};  // of an even and an odd block
+  const double dmax = first > 0 ? 0.0 : (scale ? *scale : largest_diagonal(A, n));
   for (int e = tid; e < T.rows * T.cols; e += kIT) {
     const int i = i0 + e / T.cols, j = j0 + e % T.cols;
-    double v = i == j ? 1.0 : 0.0;
-    if (i < n && j < n) {
-      v = __ldcg(A + (int64_t)i * n + j);
-      if (i == j) v = v > zero_tol * dmax ? v + shift * dmax : dmax;
-    }
-    ff_split(v, B[e].x, B[e].y);
+    if (first == 0)
+      B[e] = ff_pair(regularised(A, n, i, j, dmax, zero_tol, shift));
+    else
+      B[e] = i < n && j < n ? A2[(int64_t)i * n + j] : make_float2(i == j ? 1.f : 0.f, 0.f);
   }
-  __syncthreads();
   // raw rows of block k at the tile's columns, for every tile that holds them
   auto publish = [&](int k) {
     const int k0 = k * kB;
     if (k0 < i0 || k0 >= i0 + T.rows) return;
     for (int e = tid; e < kB * T.cols; e += kIT) {
       const int l = e / T.cols, j = j0 + e % T.cols;
-      if (j < n) {
-        const float2 v = B[(k0 - i0 + l) * T.cols + e % T.cols];
-        __stcg(ph[k & 1] + (int64_t)l * n + j, v.x);
-        __stcg(pl[k & 1] + (int64_t)l * n + j, v.y);
-      }
+      if (j < n) rows[k & 1][(int64_t)l * n + j] = B[(k0 - i0 + l) * T.cols + e % T.cols];
     }
   };
-  publish(0);
   const int steps = (n + kB - 1) / kB;
-  uint32_t target = gridDim.x;
-  bool ok = grid_barrier(bar, target, &s_ok);
-  for (int k = 0; k < steps && ok; ++k) {
+  __syncthreads();
+  if (first == 0 && !scale) publish(0);
+  __syncthreads();
+  for (int k = first; k < last; ++k) {
     const int k0 = k * kB;
-    const float *rh = ph[k & 1], *rl = pl[k & 1];
+    const float2* rk = rows[k & 1];
     auto raw = [&](int l, int j) {  // B[k0 + l][j]
-      return j < n ? make_float2(__ldcg(rh + (int64_t)l * n + j), __ldcg(rl + (int64_t)l * n + j))
-                   : make_float2(k0 + l == j ? 1.f : 0.f, 0.f);
+      return j < n && k0 + l < n ? __ldcg(rk + (int64_t)l * n + j) : make_float2(k0 + l == j ? 1.f : 0.f, 0.f);
     };
-    {
-      const int l = tid / kB, c = tid % kB;
-      M[0][l][c] = raw(l, k0 + c);
-    }
+    const int pi = tid / kB, pj = tid % kB;  // the thread's element of the pivot block
+    const float2 own = raw(pi, k0 + pj);
+    M[0][pi][pj] = own;
     for (int e = tid; e < kB * T.cols; e += kIT) {
       const float2 v = raw(e / T.cols, j0 + e % T.cols);
       RJ[e] = (double)v.x + (double)v.y;
     }
-    for (int e = tid; e < kB * T.rows; e += kIT) {
-      const int l = e / T.rows, i = i0 + e % T.rows;
-      float2 v = raw(l, i);
-      if (i < k0) v = make_float2(-v.x, -v.y);
-      RI[(e % T.rows) * kB + l] = v;
+    for (int r0 = 0; r0 < T.rows; r0 += 64) {  // 64 rows, a quarter of the block's columns a thread
+      const int r = r0 + tid % 64, i = i0 + r, l0 = tid / 64 * 4;
+      if (r >= T.rows) continue;
+      float2 v[4];
+#pragma unroll
+      for (int l = 0; l < 4; ++l) v[l] = raw(l0 + l, i);
+      const float sg = i < k0 ? -1.f : 1.f;
+      float4* q = reinterpret_cast<float4*>(RI + r * kB + l0);
+      q[0] = make_float4(sg * v[0].x, sg * v[0].y, sg * v[1].x, sg * v[1].y);
+      q[1] = make_float4(sg * v[2].x, sg * v[2].y, sg * v[3].x, sg * v[3].y);
     }
     __syncthreads();
     // P: Gauss-Jordan of the pivot block, one element per thread
-    {
-      const int i = tid / kB, j = tid % kB;
 #pragma unroll 1
-      for (int p = 0; p < kB; ++p) {
-        const float2(*S)[kB + 1] = M[p & 1];
-        const float2 r = ff_recip(S[p][p]);
-        const float2 pj = j == p ? r : ff_mul(S[p][j], r);  // row p of the new state
-        float2 v = pj;
-        if (i != p) {
-          const float2 c = ff_mul(S[i][p], pj);
-          const float2 b = j == p ? make_float2(0.f, 0.f) : S[i][j];
-          ff_sub(b.x, b.y, c.x, c.y, v.x, v.y);
-        }
-        M[(p + 1) & 1][i][j] = v;
-        __syncthreads();
+    for (int p = 0; p < kB; ++p) {
+      const float2(*S)[kB + 1] = M[p & 1];
+      const float2 r = ff_recip(S[p][p]);
+      const float2 row = pj == p ? r : ff_mul(S[p][pj], r);  // row p of the new state
+      float2 v = row;
+      if (pi != p) {
+        const float2 c = ff_mul(S[pi][p], row);
+        const float2 b = pj == p ? make_float2(0.f, 0.f) : S[pi][pj];
+        ff_sub(b.x, b.y, c.x, c.y, v.x, v.y);
       }
+      M[(p + 1) & 1][pi][pj] = v;
+      __syncthreads();
     }
     static_assert(kB % 2 == 0 && kIT == kB * kB, "P ends in M[0], one element per thread");
     // the pairs lose the block's condition number; one step
@@ -189,34 +180,31 @@ __global__ void __launch_bounds__(kIT, 1) coarse_inverse_kernel(double* __restri
     // ill-conditioned for that (rotations of one- or two-node aggregates leave
     // pivots at the level of the shift) is inverted in FP64, ~15 us slower.
     // P stays in FP64 for P B_KJ.
-    {
-      const int i = tid / kB, j = tid % kB;
-      const float2 b = raw(i, k0 + j), p0 = M[0][i][j];
-      D[0][i][j] = (double)b.x + (double)b.y;
-      const double p64 = (double)p0.x + (double)p0.y;
-      D[1][i][j] = p64;
-      __syncthreads();
-      double e = i == j ? 1.0 : 0.0;
+    const float2 pp = M[0][pi][pj];
+    const double p64 = (double)pp.x + (double)pp.y;
+    D[0][pi][pj] = (double)own.x + (double)own.y;
+    D[1][pi][pj] = p64;
+    __syncthreads();
+    double e = pi == pj ? 1.0 : 0.0;
 #pragma unroll
-      for (int q = 0; q < kB; ++q) e -= D[0][i][q] * D[1][q][j];
-      M[1][i][j].x = (float)e;
-      if (!__syncthreads_or(!(fabs(e) <= kIllResidual))) {
-        float c = 0.f;
+    for (int q = 0; q < kB; ++q) e -= D[0][pi][q] * D[1][q][pj];
+    M[1][pi][pj].x = (float)e;
+    if (!__syncthreads_or(!(fabs(e) <= kIllResidual))) {
+      float c = 0.f;
 #pragma unroll
-        for (int q = 0; q < kB; ++q) c += M[0][i][q].x * M[1][q][j].x;
-        D[0][i][j] = p64 + (double)c;
-      } else {
+      for (int q = 0; q < kB; ++q) c += M[0][pi][q].x * M[1][q][pj].x;
+      D[0][pi][pj] = p64 + (double)c;
+    } else {
 #pragma unroll 1
-        for (int p = 0; p < kB; ++p) {
-          const double(*S)[kB + 1] = D[p & 1];
-          const double r = 1.0 / S[p][p];
-          const double pj = j == p ? r : S[p][j] * r;
-          D[(p + 1) & 1][i][j] = i == p ? pj : (j == p ? 0.0 : S[i][j]) - S[i][p] * pj;
-          __syncthreads();
-        }
+      for (int p = 0; p < kB; ++p) {
+        const double(*S)[kB + 1] = D[p & 1];
+        const double r = 1.0 / S[p][p];
+        const double row = pj == p ? r : S[p][pj] * r;
+        D[(p + 1) & 1][pi][pj] = pi == p ? row : (pj == p ? 0.0 : S[pi][pj]) - S[pi][p] * row;
+        __syncthreads();
       }
-      __syncthreads();
     }
+    __syncthreads();
     const double(*P)[kB + 1] = D[0];
     // P B_KJ (columns of the pivot block itself: P)
     for (int e = tid; e < kB * T.cols; e += kIT) {
@@ -239,85 +227,105 @@ __global__ void __launch_bounds__(kIT, 1) coarse_inverse_kernel(double* __restri
         float2 pr[kB];
 #pragma unroll
         for (int l = 0; l < kB; ++l) pr[l] = PR[l * T.cols + c];
-        for (int r = g; r < T.rows; r += groups) {
-          const int i = i0 + r;
-          float2 v;
-          if (i >= k0 && i < k0 + kB) {
-            v = PR[(i - k0) * T.cols + c];
-          } else {
-            const float4* ci = reinterpret_cast<const float4*>(RI + r * kB);
-            float sh = 0.f, sl = 0.f;
+        constexpr int R = 2;  // rows at once: each row is one chain of additions
+        for (int r0 = g; r0 < T.rows; r0 += R * groups) {
+          float sh[R], sl[R];
+          int r[R];
 #pragma unroll
-            for (int l = 0; l < kB; l += 2) {
-              const float4 q = ci[l / 2];
-              ff_fma_acc(sh, sl, q.x, q.y, pr[l].x, pr[l].y);
-              ff_fma_acc(sh, sl, q.z, q.w, pr[l + 1].x, pr[l + 1].y);
-            }
-            const float2 b = jk ? make_float2(0.f, 0.f) : B[r * T.cols + c];
-            ff_sub(b.x, b.y, sh, sl, v.x, v.y);
+          for (int m = 0; m < R; ++m) {
+            r[m] = r0 + m * groups < T.rows ? r0 + m * groups : r0;
+            sh[m] = sl[m] = 0.f;
           }
-          B[r * T.cols + c] = v;
+#pragma unroll
+          for (int l = 0; l < kB; l += 2)
+#pragma unroll
+            for (int m = 0; m < R; ++m) {
+              const float4 q = reinterpret_cast<const float4*>(RI + r[m] * kB)[l / 2];
+              ff_fma_acc(sh[m], sl[m], q.x, q.y, pr[l].x, pr[l].y);
+              ff_fma_acc(sh[m], sl[m], q.z, q.w, pr[l + 1].x, pr[l + 1].y);
+            }
+          float2 v[R];
+#pragma unroll
+          for (int m = 0; m < R; ++m) {
+            const int i = i0 + r[m];
+            const float2 b = jk ? make_float2(0.f, 0.f) : B[r[m] * T.cols + c];
+            ff_sub(b.x, b.y, sh[m], sl[m], v[m].x, v[m].y);
+            if (i >= k0 && i < k0 + kB) v[m] = PR[(i - k0) * T.cols + c];
+          }
+#pragma unroll
+          for (int m = 0; m < R; ++m) B[r[m] * T.cols + c] = v[m];
         }
       }
     }
-    if (k + 1 < steps) {
-      __syncthreads();
-      publish(k + 1);
-      target += gridDim.x;
-      ok = grid_barrier(bar, target, &s_ok);
-    }
+    __syncthreads();
+    if (k + 1 < steps) publish(k + 1);
+    __syncthreads();  // a launch of several steps has one CTA: it reads its own rows
   }
-  __syncthreads();
   for (int e = tid; e < T.rows * T.cols; e += kIT) {
     const int i = i0 + e / T.cols, j = j0 + e % T.cols;
-    // a wait that ran out must not leave a plausible inverse
-    if (i < n && j < n) A[(int64_t)i * n + j] = ok ? (double)B[e].x + (double)B[e].y : (double)NAN;
+    if (i >= n || j >= n) continue;
+    if (last == steps)
+      A[(int64_t)i * n + j] = (double)B[e].x + (double)B[e].y;
+    else
+      A2[(int64_t)i * n + j] = B[e];
   }
 }
 
 }  // namespace
 
-// The smallest tiles (most CTAs) whose grid fits on the SMs, one CTA each.
-// Up to 48 unknowns one CTA saves the barriers.
+// Tile of an inversion of 'panels' pivot blocks on 'sms' SMs, one CTA each:
+// the least work per step (cycles: 1.6 an entry of the tile, 128 a column for
+// P B_KJ at two FP64 products a cycle, 6 a row or column loaded, 6000 for the
+// rest).  Narrow tiles save FP64 work: 612 unknowns in 64 x 64 tiles took 0.90
+// ms, in 208 x 16 ones 0.82.  Up to 48 unknowns one CTA does all steps in one
+// launch.
+static Tile pick_tile(int panels, int sms) {
+  Tile best{panels * kB, panels * kB, 1};
+  if (panels <= 3) return best;
+  double cost = 1e300;
+  for (int a = 1; a <= panels; ++a)
+    for (int b = 1; b <= panels; ++b) {
+      const Tile t{a * kB, b * kB, (int)ceil_div(panels, b)};
+      if (t.cols > kIT || tile_smem(t) > kSmemMax) continue;
+      const double waves = (double)ceil_div(ceil_div(panels, a) * t.gc, sms);
+      const double c = waves * (1.6 * t.rows * t.cols + 128.0 * t.cols + 6.0 * (t.rows + t.cols) + 6000);
+      if (c < cost) {
+        cost = c;
+        best = t;
+      }
+    }
+  return best;
+}
+
 int coarse_inverse(const CoarseDev& C, double zero_tol, double shift, cudaStream_t st) {
   const int n = C.nc, panels = (int)ceil_div(n, kB);
-  Tile best{0, 0, 0};
-  int grid = 0;
-  if (panels <= 3) {
-    best = Tile{panels * kB, panels * kB, 1};
-    grid = 1;
-  } else {
-    int area = 1 << 30;
-    for (int a = 1; a * kB <= kTileMax; ++a)
-      for (int b = 1; b * kB <= kTileMax; ++b) {
-        const int gr = (int)ceil_div(panels, a), gc = (int)ceil_div(panels, b);
-        if (gr * gc > kSMs) continue;
-        // equal areas: the squarer tile (shorter panels to load)
-        if (a * b < area || (a * b == area && a + b < (best.rows + best.cols) / kB)) {
-          area = a * b;
-          best = Tile{a * kB, b * kB, gc};
-          grid = gr * gc;
-        }
-      }
-    if (grid == 0) return GFEA_ERR_ARG;
+  const Tile t = pick_tile(panels, kSMs);
+  const int grid = (int)ceil_div(panels * kB, t.rows) * t.gc;
+  const size_t smem = tile_smem(t);
+  GFEA_CUDA_TRY(allow_smem(coarse_inverse_kernel, kSmemMax));
+  // the published rows: pairs over (rowph, rowpl) for even blocks, (colph, colpl) for odd ones
+  float2 *rows0 = reinterpret_cast<float2*>(C.rowph), *rows1 = reinterpret_cast<float2*>(C.colph);
+  double* scale = grid > 1 ? reinterpret_cast<double*>(C.pinvh) : nullptr;
+  if (scale) {
+    coarse_inverse_start_kernel<<<(int)ceil_div(n, kIT), kIT, 0, st>>>(C.Ac, n, rows0, scale, zero_tol, shift);
+    GFEA_LAUNCH_CHECK();
   }
-  const size_t smem = tile_smem(best);
-  GFEA_CUDA_TRY(allow_smem(coarse_inverse_kernel, tile_smem(Tile{kTileMax, kTileMax, 1})));
-  uint32_t* bar = reinterpret_cast<uint32_t*>(C.pinvh);
-  GFEA_CUDA_TRY(cudaMemsetAsync(bar, 0, sizeof(uint32_t), st));
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = dim3(grid);
   cfg.blockDim = dim3(kIT);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = st;
   cudaLaunchAttribute at[1];
-  at[0].id = cudaLaunchAttributeCooperative;
-  at[0].val.cooperative = 1;
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = at;
-  cfg.numAttrs = grid > 1 ? 1 : 0;
-  GFEA_CUDA_TRY(cudaLaunchKernelEx(&cfg, coarse_inverse_kernel, C.Ac, n, best, C.rowph, C.rowpl, C.colph, C.colpl,
-                                   bar, zero_tol, shift));
-  GFEA_LAUNCH_CHECK();
+  cfg.numAttrs = scale ? 1 : 0;
+  const int each = scale ? 1 : panels;  // one CTA takes every step in one launch
+  for (int k = 0; k < panels; k += each) {
+    GFEA_CUDA_TRY(cudaLaunchKernelEx(&cfg, coarse_inverse_kernel, C.Ac, n, t, rows0, rows1, (const double*)scale, k,
+                                     k + each, zero_tol, shift));
+    GFEA_LAUNCH_CHECK();
+  }
   return GFEA_OK;
 }
 

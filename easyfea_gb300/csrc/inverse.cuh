@@ -7,7 +7,8 @@ namespace gfea {
 
 // C.Ac (nc x nc, SPD) regularised -- a diagonal entry at most zero_tol times
 // the largest is replaced by it, the others shifted by 'shift' times it --
-// and inverted in place, in one cooperative launch on st.
+// and inverted in place on st: a launch per 16 unknowns, none of which waits on
+// another CTA.
 int coarse_inverse(const CoarseDev& C, double zero_tol, double shift, cudaStream_t st);
 
 }  // namespace gfea

@@ -63,3 +63,12 @@ def test_shared_memory_is_opted_into_on_every_device(run, case, kernel):
         assert any(n.startswith(kernel) for n in names(s)), names(s)
         assert not refused(s)
     assert names(out[0]) == names(out[1])
+
+
+@pytest.mark.parametrize("sms", [152, 100, 16])
+@pytest.mark.parametrize("aggregates", [40, 250])
+def test_coarse_inverse_needs_no_co_resident_grid(run, sms, aggregates):
+    """240 and 1,500 coarse unknowns on a device or an MPS share of fewer SMs."""
+    (s,) = run({**BOX, "nodes": 100000, "coarse": aggregates, "sms": sms})
+    inverse = [line for line in s["launches"] if line.startswith("coarse_inverse")]
+    assert inverse and not any("cooperative" in line or "refused" in line for line in inverse)
