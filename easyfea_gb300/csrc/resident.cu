@@ -1028,7 +1028,12 @@ int launch(const ResidentProblem<T>& P, const ResidentGeom& g, cudaStream_t st) 
   a[0].val.cooperative = 1;
   cfg.attrs = a;
   cfg.numAttrs = g.grid > 1 ? 1 : 0;
-  GFEA_CUDA_TRY(cudaLaunchKernelEx(&cfg, kern, P, g));
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, kern, P, g);
+  if (e == cudaErrorCooperativeLaunchTooLarge) {
+    cudaGetLastError();  // not sticky: taken back
+    return kResidentRefused;
+  }
+  GFEA_CUDA_TRY(e);
   GFEA_LAUNCH_CHECK();
   return GFEA_OK;
 }

@@ -42,6 +42,9 @@ struct ResidentGeom {
 template <typename T>
 bool resident_geom(int D, int64_t Nn, int64_t n_pairs, int nc, int n_agg, int sms, ResidentGeom* g);
 
+// GFEA_OK, an error, or kResidentRefused: the grid does not fit on the SMs this
+// context has (nothing was launched).
+constexpr int kResidentRefused = -1;
 template <typename T>
 int resident_launch(int D, const ResidentProblem<T>& P, const ResidentGeom& g, cudaStream_t st);
 

@@ -2040,6 +2040,11 @@ int fetch(Scal* h, PcgWork& w, cudaStream_t st) {
 // that is not staged (its tiles would fit in half of the L2), host checks left
 // to the library, and nothing that needs the iteration's launches one by one
 // (kernel timing, a first solve that tunes the SpMV, the direct-launch entry).
+//
+// Its CTAs, one per SM, must all run at once: the grid is bounded by the
+// device's SMs (an MPS share's, where the context has one), and a launch that
+// is refused all the same (a green context) leaves the solve to the
+// multi-kernel iteration.
 template <typename T>
 bool use_resident(const gfea_system* s, const gfea_pcg_opts* o, const PcgWork& w, bool direct_only, ResidentGeom* g) {
   if (direct_only || !w.box || o->check_every > 0 || prof().on.load()) return false;
@@ -2056,8 +2061,13 @@ bool use_resident(const gfea_system* s, const gfea_pcg_opts* o, const PcgWork& w
   // latency (24 served requests: 55 ms with full-size grids, 39 ms with a
   // share each, 48 ms with the multi-kernel iteration).
   const int active = std::min(std::max(active_solves().load(), 1), 4);
+  int dev = 0, sms = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess ||
+      cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
+    return false;
+  sms = std::min(sms, kSMs);  // the packets' room
   return resident_geom<T>(s->dof_n, s->n_nodes, s->n_pairs, w.coarse ? w.C.nc : 0, w.coarse ? w.C.n_agg : 0,
-                          kSMs / active, g);
+                          std::max(sms / active, 1), g);
 }
 
 // PCG in T precision with reliable updates (FP64 residual replacement):
@@ -2155,15 +2165,17 @@ int refine_solve(const gfea_system* s, const double* b, double* x, const gfea_pc
     P.max_upd = o->max_refine > 0 ? o->max_refine : 200;
     GFEA_CUDA_TRY(cudaMemsetAsync(P.box, 0, kResidentBox / (kSMs * kSMs) * geom.grid * geom.grid, st));
     e = resident_launch<T>(s->dof_n, P, geom, st);
-    if (e) return e;
-    GFEA_CUDA_TRY(cudaMemcpyAsync(res, P.out, sizeof(*res), cudaMemcpyDeviceToHost, st));
-    GFEA_CUDA_TRY(cudaStreamSynchronize(st));
-    if (getenv("GFEA_DEBUG"))
-      fprintf(stderr, "[gfea pcg%d] resident: %d CTAs, iterations %d, updates %d, status %d, rel residual %.3e, %.2f ms\n",
-              fp64 ? 64 : 32, geom.grid, res->iterations, res->refinements, res->status,
-              res->rel_residual,
-              std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t_start).count());
-    return res->status;
+    if (e == GFEA_OK) {
+      GFEA_CUDA_TRY(cudaMemcpyAsync(res, P.out, sizeof(*res), cudaMemcpyDeviceToHost, st));
+      GFEA_CUDA_TRY(cudaStreamSynchronize(st));
+      if (getenv("GFEA_DEBUG"))
+        fprintf(stderr, "[gfea pcg%d] resident: %d CTAs, iterations %d, updates %d, status %d, rel residual %.3e, %.2f ms\n",
+                fp64 ? 64 : 32, geom.grid, res->iterations, res->refinements, res->status,
+                res->rel_residual,
+                std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t_start).count());
+      return res->status;
+    }
+    if (e != kResidentRefused) return e;
   }
   e = launch_bjacobi<T>(s, w, st);
   if (e) return e;

@@ -72,3 +72,23 @@ def test_coarse_inverse_needs_no_co_resident_grid(run, sms, aggregates):
     (s,) = run({**BOX, "nodes": 100000, "coarse": aggregates, "sms": sms})
     inverse = [line for line in s["launches"] if line.startswith("coarse_inverse")]
     assert inverse and not any("cooperative" in line or "refused" in line for line in inverse)
+
+
+def resident_ctas(step):
+    return [int(line.split()[2]) for line in step["launches"] if line.startswith("resident_kernel")]
+
+
+@pytest.mark.parametrize("sms", [152, 100, 16])
+def test_resident_grid_fits_the_device(run, sms):
+    (s,) = run({**BOX, "nodes": 5000, "sms": sms})
+    assert s["status"] in (0, 5) and not refused(s)
+    assert resident_ctas(s) and max(resident_ctas(s)) <= sms or "apply_kernel" in names(s)
+
+
+def test_refused_cooperative_launch_leaves_the_multi_kernel_iteration(run):
+    """A context of fewer SMs than the device reports (a green context)."""
+    (s,) = run({**BOX, "coop_limit": 60})
+    assert s["status"] == 5 == s["result"]  # the recorded iteration stops at once
+    assert [line.split()[0] for line in refused(s)] == ["resident_kernel"]
+    after = names(s)[names(s).index("resident_kernel") + 1:]
+    assert "bjacobi_kernel" in after and any(n.startswith("apply") for n in after)
