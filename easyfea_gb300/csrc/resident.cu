@@ -29,8 +29,9 @@
 // packets (the sums s, x after an update) is ordered by fences around the
 // exchange of the partial sums (1).  Every CTA adds the partials in the same order, so all take the same
 // decisions (convergence, updates, stopping) without the host.  The launch is
-// cooperative (the CTAs are co-resident); every poll is bounded: after 2 s
-// the solve ends with GFEA_ERR_TIMEOUT.
+// cooperative (the CTAs are co-resident); every poll is bounded: after 2 s (a
+// context suspended that long) the launch ends and reports it, and the host
+// goes on with the multi-kernel iteration, which waits for nothing.
 //
 // Bound: latency (three exchanges of ~2 us, the halo, the serial chains
 // between them); in FP64 3D also the FP64 pipe (27 x 9 products per node: 5 us
@@ -103,11 +104,11 @@ struct Packet<double> {
 struct Deadline {
   uint64_t t0 = 0;
   uint32_t n = 0;
-  __device__ __forceinline__ bool expired(volatile int* abort) {
+  __device__ __forceinline__ bool expired(volatile int* abort, uint64_t limit_ns) {
     if ((++n & 255u) != 0) return false;
     const uint64_t t = global_ns();
     if (t0 == 0) t0 = t;
-    if (*abort || t - t0 > kWaitLimitNs) {
+    if (*abort || t - t0 > limit_ns) {
       *abort = 1;
       return true;
     }
@@ -117,12 +118,12 @@ struct Deadline {
 
 // The value of packet p once it carries 'tag' (0 when the wait ran out).
 template <typename T>
-__device__ __forceinline__ T await_packet(const T* p, uint32_t tag, volatile int* abort) {
+__device__ __forceinline__ T await_packet(const T* p, uint32_t tag, volatile int* abort, uint64_t limit_ns) {
   uint32_t t;
   T v = Packet<T>::load(p, &t);
   Deadline d;
   while (t != tag) {
-    if (d.expired(abort)) return 0;
+    if (d.expired(abort, limit_ns)) return 0;
     v = Packet<T>::load(p, &t);
   }
   return v;
@@ -140,15 +141,17 @@ struct Team {
   uint32_t number;     // exchanges so far
   double (*shw)[kRW];  // warp sums
   double* res;         // reduced values
-  volatile int* abort;
+  volatile int* abort; // a wait of this CTA ran out
+  int* ok;             // its verdict at the last exchange, the same for every thread
+  uint64_t limit_ns;
 };
 
 // Exchange of NV sums (w: warp sums, valid in lane 0).  Value k belongs to
 // warp k, which publishes the CTA's sum and adds all CTAs' in a fixed order;
 // the other warps run meanwhile(thread, threads); thread 0 then runs
 // f(totals), whose shared-memory results every thread sees.  FENCE: writes
-// before the exchange (any CTA) are visible after it (through ld.cg).  False
-// when a wait ran out.
+// before the exchange (any CTA) are visible after it (through ld.cg).  False,
+// for every thread of the CTA, when a wait ran out before.
 template <int NV, bool FENCE, typename M, typename F>
 __device__ __forceinline__ bool exchange(Team& t, const double (&w)[NV], M meanwhile, F f) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -188,7 +191,7 @@ __device__ __forceinline__ bool exchange(Team& t, const double (&w)[NV], M meanw
         }
       }
       Deadline d;
-      while (wait && !d.expired(t.abort)) {
+      while (wait && !d.expired(t.abort, t.limit_ns)) {
         wait = false;
 #pragma unroll
         for (int u = 0; u < U; ++u) {
@@ -213,9 +216,12 @@ __device__ __forceinline__ bool exchange(Team& t, const double (&w)[NV], M meanw
     meanwhile((int)threadIdx.x - NV * 32, kRT - NV * 32);
   }
   __syncthreads();
-  if (threadIdx.x == 0) f(t.res);
+  if (threadIdx.x == 0) {
+    f(t.res);
+    *t.ok = *t.abort == 0;  // one reading for all: a thread ahead may give up while another reads
+  }
   __syncthreads();
-  return *t.abort == 0;
+  return *t.ok != 0;
 }
 
 template <bool FENCE>
@@ -343,7 +349,7 @@ __global__ void __launch_bounds__(kRT, 1) resident_kernel(ResidentProblem<T> P, 
   extern __shared__ __align__(16) unsigned char smem[];
   __shared__ double s_w[4][kRW];
   __shared__ double s_res[4];
-  __shared__ int s_abort, s_scan[kRW], s_range[2], s_nseg;
+  __shared__ int s_abort, s_ok, s_scan[kRW], s_range[2], s_nseg;
   __shared__ uint32_t s_bits[kAggWords];
   __shared__ int s_base[kAggWords];
   __shared__ Ctl ctl;
@@ -382,7 +388,7 @@ __global__ void __launch_bounds__(kRT, 1) resident_kernel(ResidentProblem<T> P, 
     s_range[1] = -1;
     s_nseg = 0;
   }
-  Team team{P.box, 0, s_w, s_res, &s_abort};
+  Team team{P.box, 0, s_w, s_res, &s_abort, &s_ok, P.wait_ns};
 
   // ---- own nodes a0 .. a0 + n ---------------------------------------------
   const int64_t a0 = min((int64_t)blockIdx.x * geom.npc, S.Nn);
@@ -651,7 +657,7 @@ __global__ void __launch_bounds__(kRT, 1) resident_kernel(ResidentProblem<T> P, 
             for (int u = 0; u < U; ++u) {
               const int i = i0 + u * kRT;
               if (i < cnt) {
-                if (tag[u] != p_number) v[u] = await_packet<T>(src[u], p_number, &s_abort);
+                if (tag[u] != p_number) v[u] = await_packet<T>(src[u], p_number, &s_abort, P.wait_ns);
                 pl_s[i] = v[u];
               }
             }
@@ -663,7 +669,7 @@ __global__ void __launch_bounds__(kRT, 1) resident_kernel(ResidentProblem<T> P, 
       auto p_at = [&](int slot, int j) -> T {
         if (pl_s) return pl_s[lidx_s[slot] * D + j];
         const int64_t c = (int64_t)__ldg(NBg + slot) * D + j;
-        return solo ? p_s[c] : await_packet<T>(P.p + 2 * c, p_number, &s_abort);
+        return solo ? p_s[c] : await_packet<T>(P.p + 2 * c, p_number, &s_abort, P.wait_ns);
       };
       if constexpr (sizeof(T) == 4) {
         constexpr int LA = G - G % D, NPP = LA / D;
@@ -955,7 +961,7 @@ __global__ void __launch_bounds__(kRT, 1) resident_kernel(ResidentProblem<T> P, 
         [&](int t, int nt) {  // the own aggregates' corrections
           if (!solo)
             for (int i = t; i < s_nseg * nr; i += nt)
-              ecl_s[i] = await_packet<T>(P.ec + 2 * (seg_agg[i / nr] * nr + i % nr), ec_number, &s_abort);
+              ecl_s[i] = await_packet<T>(P.ec + 2 * (seg_agg[i / nr] * nr + i % nr), ec_number, &s_abort, P.wait_ns);
         },
         [&](const double* o) {
           const double rz = o[0], rr = o[1];
@@ -1002,16 +1008,44 @@ __global__ void __launch_bounds__(kRT, 1) resident_kernel(ResidentProblem<T> P, 
     }
     if (solo || !pl_s) __syncthreads();
   }
+  if (!ok && tid == 0) P.out->timed_out = 1;
   if (blockIdx.x == 0 && tid == 0) {
     gfea_pcg_result res{};
-    res.status = ok ? ctl.status : GFEA_ERR_TIMEOUT;
+    res.status = ctl.status;
     res.iterations = ctl.iters;
     res.refinements = ctl.updates;
     const bool rel = ctl.bb > 0 && ctl.status != GFEA_ERR_SINGULAR;
     res.rel_residual = rel ? sqrt(ctl.rr_true / ctl.bb) : 0.0;
     res.floor_rel = rel ? sqrt(ctl.floor2 / ctl.bb) : 0.0;
-    *P.out = res;
+    P.out->res = res;
   }
+}
+
+// Two CTAs, of which the second takes part in an exchange and publishes a
+// packet, or leaves at once: the first one's waits end or run out.
+__device__ __align__(16) double selftest_box[2 * 4 * 2 * 2 * 2 + 2];
+__device__ int32_t selftest_exchanged;
+
+__global__ void __launch_bounds__(kRT) exchange_selftest_kernel(uint64_t limit_ns, int present) {
+  __shared__ double s_w[4][kRW];
+  __shared__ double s_res[4];
+  __shared__ int s_abort, s_ok;
+  if (blockIdx.x == 1 && !present) return;
+  if (threadIdx.x == 0) s_abort = 0;
+  __syncthreads();
+  Team team{selftest_box, 0, s_w, s_res, &s_abort, &s_ok, limit_ns};
+  float* packet = reinterpret_cast<float*>(selftest_box + 2 * 4 * 2 * 2 * 2);
+  const double w[1] = {1.0};
+  double total = 0;
+  bool ok = exchange<1, true>(team, w, [](int, int) {}, [&](const double* o) { total = o[0]; });
+  if (blockIdx.x == 1) {
+    if (threadIdx.x == 0) Packet<float>::store(packet, 3.f, 7);
+    return;
+  }
+  const float v = await_packet<float>(packet, 7, &s_abort, limit_ns);
+  __syncthreads();
+  ok = ok && s_abort == 0;
+  if (threadIdx.x == 0) selftest_exchanged = ok && total == 2.0 * kRW && v == 3.f ? GFEA_OK : GFEA_ERR_TIMEOUT;
 }
 
 template <int D, int G, typename T>
@@ -1093,3 +1127,30 @@ template int resident_launch<float>(int, const ResidentProblem<float>&, const Re
 template int resident_launch<double>(int, const ResidentProblem<double>&, const ResidentGeom&, cudaStream_t);
 
 }  // namespace gfea
+
+using namespace gfea;
+
+extern "C" int gfea_selftest_exchange(int32_t limit_us, int32_t present, int32_t* status_host, void* stream) {
+  if (!status_host || limit_us < 1 || limit_us > 1000000) return GFEA_ERR_ARG;
+  cudaStream_t st = static_cast<cudaStream_t>(stream);
+  const int32_t unset = -1;
+  void* box = nullptr;
+  GFEA_CUDA_TRY(cudaGetSymbolAddress(&box, selftest_box));
+  GFEA_CUDA_TRY(cudaMemsetAsync(box, 0, sizeof(selftest_box), st));
+  GFEA_CUDA_TRY(cudaMemcpyToSymbolAsync(selftest_exchanged, &unset, sizeof(int32_t), 0, cudaMemcpyHostToDevice, st));
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(2);
+  cfg.blockDim = dim3(kRT);
+  cfg.stream = st;
+  cudaLaunchAttribute a[1];
+  a[0].id = cudaLaunchAttributeCooperative;
+  a[0].val.cooperative = 1;
+  cfg.attrs = a;
+  cfg.numAttrs = 1;
+  GFEA_CUDA_TRY(cudaLaunchKernelEx(&cfg, exchange_selftest_kernel, (uint64_t)limit_us * 1000ull, (int)(present != 0)));
+  GFEA_LAUNCH_CHECK();
+  GFEA_CUDA_TRY(cudaMemcpyFromSymbolAsync(status_host, selftest_exchanged, sizeof(int32_t), 0, cudaMemcpyDeviceToHost,
+                                          st));
+  GFEA_CUDA_TRY(cudaStreamSynchronize(st));
+  return GFEA_OK;
+}

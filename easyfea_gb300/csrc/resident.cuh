@@ -9,6 +9,12 @@
 
 namespace gfea {
 
+struct ResidentOut {
+  gfea_pcg_result res;
+  int32_t timed_out;  // a wait ran out in some CTA: x holds the updates so far, 'res' is void
+  int32_t pad;
+};
+
 // One solve.  The scratch is the multi-kernel PCG's workspace.
 template <typename T>
 struct ResidentProblem {
@@ -21,7 +27,8 @@ struct ResidentProblem {
   T* ec;              // packets of the coarse correction (2 nc values)
   int coarse;         // two-level preconditioner
   double* box;        // packets of the partial sums (zero at launch)
-  gfea_pcg_result* out;
+  ResidentOut* out;   // zero at launch
+  uint64_t wait_ns;   // limit of every wait
   double rtol, delta2;
   int max_iters, max_upd;
 };

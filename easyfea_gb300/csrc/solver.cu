@@ -2158,7 +2158,9 @@ int refine_solve(const gfea_system* s, const double* b, double* x, const gfea_pc
     P.ec = w.coarse ? reinterpret_cast<T*>(w.C.rcp + 4 * (size_t)w.C.nc) : nullptr;
     P.coarse = w.coarse ? 1 : 0;
     P.box = reinterpret_cast<double*>(w.box);
-    P.out = reinterpret_cast<gfea_pcg_result*>(w.sc);
+    static_assert(sizeof(ResidentOut) <= sizeof(Scal), "the scalar record's place");
+    P.out = reinterpret_cast<ResidentOut*>(w.sc);
+    P.wait_ns = kWaitLimitNs;
     P.rtol = o->rtol;
     P.delta2 = delta2;
     P.max_iters = o->max_iters;
@@ -2166,16 +2168,26 @@ int refine_solve(const gfea_system* s, const double* b, double* x, const gfea_pc
     GFEA_CUDA_TRY(cudaMemsetAsync(P.box, 0, kResidentBox / (kSMs * kSMs) * geom.grid * geom.grid, st));
     e = resident_launch<T>(s->dof_n, P, geom, st);
     if (e == GFEA_OK) {
-      GFEA_CUDA_TRY(cudaMemcpyAsync(res, P.out, sizeof(*res), cudaMemcpyDeviceToHost, st));
+      ResidentOut out;
+      GFEA_CUDA_TRY(cudaMemcpyAsync(&out, P.out, sizeof(out), cudaMemcpyDeviceToHost, st));
       GFEA_CUDA_TRY(cudaStreamSynchronize(st));
       if (getenv("GFEA_DEBUG"))
-        fprintf(stderr, "[gfea pcg%d] resident: %d CTAs, iterations %d, updates %d, status %d, rel residual %.3e, %.2f ms\n",
-                fp64 ? 64 : 32, geom.grid, res->iterations, res->refinements, res->status,
-                res->rel_residual,
+        fprintf(stderr,
+                "[gfea pcg%d] resident: %d CTAs, iterations %d, updates %d, status %d, rel residual %.3e%s, %.2f ms\n",
+                fp64 ? 64 : 32, geom.grid, out.res.iterations, out.res.refinements, out.res.status,
+                out.res.rel_residual, out.timed_out ? ", a wait ran out" : "",
                 std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t_start).count());
-      return res->status;
+      if (!out.timed_out) {
+        *res = out.res;
+        return res->status;
+      }
+      // x is a valid initial guess (each CTA adds whole corrections to its own
+      // unknowns); what else the launch wrote is set up again
+      GFEA_CUDA_TRY(cudaMemsetAsync(w.sc, 0, sizeof(Scal), st));
+      if (w.coarse) GFEA_CUDA_TRY(cudaMemsetAsync(w.C.rcp, 0, sizeof(double) * w.C.nc * kRcCopies, st));
+    } else if (e != kResidentRefused) {
+      return e;
     }
-    if (e != kResidentRefused) return e;
   }
   e = launch_bjacobi<T>(s, w, st);
   if (e) return e;

@@ -531,6 +531,13 @@ int gfea_profile_read(double* ms_host, long long* launches_host);
  * wait runs out); the context stays usable. */
 int gfea_selftest_wait(int32_t limit_us, int32_t arrive, int32_t* status_host, void* stream);
 
+/* The same for the waits between the CTAs of a resident solve: a cooperative
+ * grid of two, of which the second takes part in an exchange of sums and
+ * publishes a packet (present != 0: *status_host = GFEA_OK) or leaves at once
+ * (*status_host = GFEA_ERR_TIMEOUT after limit_us; a solve goes on with its
+ * multi-kernel iteration then). */
+int gfea_selftest_exchange(int32_t limit_us, int32_t present, int32_t* status_host, void* stream);
+
 /* FP64 -> FP32 copy of CSR values (mixed-precision operator) */
 int gfea_cast_f64_f32(const double* src, float* dst, int64_t n, void* stream);
 

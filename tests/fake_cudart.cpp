@@ -3,7 +3,7 @@
 // refused as the real runtime refuses it (dynamic shared memory above 48 KB
 // without the kernel's attribute on the current device, a cooperative grid
 // larger than the device).  The test sets the current device and its SMs, and
-// may have the next records of a solve report a status.
+// may have a resident solve report a wait that ran out.
 #include <cuda_runtime_api.h>
 #include <cxxabi.h>
 #include <stdlib.h>
@@ -30,7 +30,7 @@ struct Scalars {
 };
 Scalars* g_scalars = nullptr;
 
-int g_result_status = -1;  // status put into the next 40- or 48-byte solve record read by the host
+bool g_timed_out = false;  // the next resident solve reports a wait that ran out
 
 struct Config {
   dim3 grid, block;
@@ -90,7 +90,7 @@ void fake_device(int device, int sms, int coop_limit) {
   g_sms = sms;
   g_coop_limit = coop_limit;
 }
-void fake_result_status(int s) { g_result_status = s; }
+void fake_timed_out(int v) { g_timed_out = v != 0; }
 void fake_clear() { g_log.clear(); }
 const char* fake_log() { return g_log.c_str(); }
 
@@ -151,10 +151,11 @@ cudaError_t cudaOccupancyMaxActiveClusters(int* n, const void*, const cudaLaunch
 }
 cudaError_t cudaMemcpyAsync(void* dst, const void* src, size_t n, cudaMemcpyKind kind, cudaStream_t) {
   memmove(dst, src, n);
-  if (kind == cudaMemcpyDeviceToHost && (n == 40 || n == 48) && g_result_status >= 0) {
-    const int32_t st = g_result_status;
-    memcpy(dst, &st, sizeof(st));
-    g_result_status = -1;
+  if (kind == cudaMemcpyDeviceToHost && (n == 32 || n == 40) && g_timed_out) {  // a result, alone or with its flag
+    const int32_t status = 9, flag = 1;
+    memcpy(dst, &status, sizeof(status));
+    if (n == 40) memcpy(static_cast<char*>(dst) + 32, &flag, sizeof(flag));
+    g_timed_out = false;
   }
   return cudaSuccess;
 }

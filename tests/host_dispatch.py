@@ -27,7 +27,7 @@ def main(fake_path, steps):
     out = []
     for s in steps:
         fake.fake_device(s.get("device", 0), s.get("sms", 152), s.get("coop_limit", s.get("sms", 152)))
-        fake.fake_result_status(s.get("result_status", -1))
+        fake.fake_timed_out(s.get("timed_out", 0))
         L.gfea_tune_mode(s.get("tune_mode", 1))
         for k in ("GFEA_STAGE_MIN_BYTES", "GFEA_RESIDENT_CTAS"):
             os.environ.pop(k, None)

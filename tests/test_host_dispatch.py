@@ -92,3 +92,11 @@ def test_refused_cooperative_launch_leaves_the_multi_kernel_iteration(run):
     assert [line.split()[0] for line in refused(s)] == ["resident_kernel"]
     after = names(s)[names(s).index("resident_kernel") + 1:]
     assert "bjacobi_kernel" in after and any(n.startswith("apply") for n in after)
+
+
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+def test_wait_that_ran_out_leaves_the_multi_kernel_iteration(run, precision):
+    (s,) = run({**BOX, "precision": precision, "timed_out": 1})
+    assert s["status"] == 5 == s["result"]  # the recorded iteration stops at once; not GFEA_ERR_TIMEOUT
+    after = names(s)[names(s).index("resident_kernel") + 1:]
+    assert "bjacobi_kernel" in after and any(n.startswith("apply") for n in after)
