@@ -757,12 +757,38 @@ __global__ void __launch_bounds__(kRT, 1) resident_kernel(ResidentProblem<T> P, 
                 for (int d = 0; d < D; ++d) acc[d] += v[d] * xv;
               }
             } else {
+              // the lane's trips to L2 are one chain: U neighbours' at once
+              // (three, and one packet of p at a time without a halo: 9,225
+              // PRISM18 nodes 10.05 ms, four 8.39, the multi-kernel iteration 9.69)
+              constexpr int U = 4;
               const T* vr = Vg + D * D * s0 + j;
-#pragma unroll 3
-              for (int k = 0; k < nb; ++k) {
-                const T xv = p_at(s0 + k, j);
+              for (int k0 = 0; k0 < nb; k0 += U) {
+                T v[U][D], xv[U];
+                const T* src[U];
+                uint32_t tag[U];
 #pragma unroll
-                for (int d = 0; d < D; ++d) acc[d] += __ldg(vr + d * W + D * k) * xv;
+                for (int u = 0; u < U; ++u) {
+                  const int k = k0 + u;
+                  const bool in = k < nb;
+                  tag[u] = p_number;
+                  xv[u] = 0;
+                  src[u] = P.p;
+                  if (in && pl_s) {
+                    xv[u] = pl_s[lidx_s[s0 + k] * D + j];
+                  } else if (in) {
+                    const int64_t c = (int64_t)__ldg(NBg + s0 + k) * D + j;
+                    src[u] = P.p + 2 * c;
+                    xv[u] = solo ? p_s[c] : Pk::load(src[u], &tag[u]);
+                  }
+#pragma unroll
+                  for (int d = 0; d < D; ++d) v[u][d] = in ? __ldg(vr + d * W + D * k) : (T)0;
+                }
+#pragma unroll
+                for (int u = 0; u < U; ++u) {
+                  if (tag[u] != p_number) xv[u] = await_packet<T>(src[u], p_number, &s_abort, P.wait_ns);
+#pragma unroll
+                  for (int d = 0; d < D; ++d) acc[d] += v[u][d] * xv[u];
+                }
               }
             }
           }
@@ -1074,10 +1100,18 @@ int launch(const ResidentProblem<T>& P, const ResidentGeom& g, cudaStream_t st) 
 
 }  // namespace
 
-// Rows per CTA: enough to keep its threads busy, few enough to use many SMs.
+// Rows per CTA: enough to keep its threads busy, few enough to use many SMs;
+// of long rows no more than 10,240 values (a HEXA8's 128 rows), by which a CTA's
+// time goes.  Shared memory: all of it.  Numberings that take the corner nodes
+// first (every quadratic 3D mesh) give the first CTAs rows of twice the average
+// length, which room for the average left to L2.  In FP64, average room and 128
+// rows -> this, beside the multi-kernel iteration's: 425 HEXA27 nodes 4.75 -> 2.44
+// ms (3.22), 2,025 8.42 -> 3.99 (6.31), 600 HEXA20 6.21 -> 3.19 (4.79), 2,025
+// PRISM18 7.68 -> 3.87 (5.60), 2,025 TETRA10 6.71 -> 3.56 (6.11).
 template <typename T>
 bool resident_geom(int D, int64_t Nn, int64_t n_pairs, int nc, int n_agg, int sms, ResidentGeom* g) {
-  const int64_t rows = sizeof(T) == 8 ? 128 : 256;
+  const double nb = (double)n_pairs / (double)Nn;
+  const int64_t rows = std::min<int64_t>(sizeof(T) == 8 ? 128 : 256, std::max<int64_t>(32, (int64_t)(10240 / (nb * D))));
   if (const char* e = getenv("GFEA_RESIDENT_CTAS"))  // fewer, larger CTAs
     if (atoi(e) > 0) sms = std::min(sms, atoi(e));
   int64_t grid = ceil_div(Nn * D, rows);
@@ -1087,13 +1121,9 @@ bool resident_geom(int D, int64_t Nn, int64_t n_pairs, int nc, int n_agg, int sm
   g->npc = (int)npc;
   g->grid = (int)ceil_div(Nn, npc);
   if (n_agg > kAggWords * 32) return false;
-  const double nb = (double)n_pairs / (double)Nn;
   const size_t fixed = Layout<T>(D, g->npc, nc, n_agg, g->grid == 1).total;
   if (fixed > kRSmemMax / 2) return false;
-  // everything resident, with a generous halo and A_c^-1's rows
-  const double want = (double)fixed + npc * nb * (1.1 * sizeof(T) * D * D + 2) +
-                      (4 + sizeof(T) * D) * std::min<double>((double)Nn, npc * nb) + 8.0 * nc * (nc / g->grid + 1) + 4096;
-  g->smem = (size_t)std::min<double>(want, (double)kRSmemMax);
+  g->smem = kRSmemMax;
   // lanes per node by the row length, as in the multi-kernel SpMV
   const double W = D * nb;
   g->lanes = D == 1 ? (W <= 10 ? 4 : 8) : (D == 2 ? (W <= 24 ? 8 : 16) : (W <= 56 ? 16 : 32));

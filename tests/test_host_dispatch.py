@@ -100,3 +100,16 @@ def test_wait_that_ran_out_leaves_the_multi_kernel_iteration(run, precision):
     assert s["status"] == 5 == s["result"]  # the recorded iteration stops at once; not GFEA_ERR_TIMEOUT
     after = names(s)[names(s).index("resident_kernel") + 1:]
     assert "bjacobi_kernel" in after and any(n.startswith("apply") for n in after)
+
+
+@pytest.mark.parametrize("nodes,degree,precision,least", [(2025, 52, "fp64", 90), (2025, 52, "mixed", 90),
+                                                          (600, 41, "fp64", 18), (2025, 24, "fp64", 40)])
+def test_long_rows_spread_over_more_ctas(run, nodes, degree, precision, least):
+    """A CTA's work goes by its stored values, and the longest rows come
+    together (corner nodes first): about 10,240 values a CTA, with all of the
+    shared memory for them."""
+    (s,) = run({**BOX, "nodes": nodes, "degree": degree, "precision": precision})
+    (line,) = [line for line in s["launches"] if line.startswith("resident_kernel")]
+    w = line.split()
+    assert least <= int(w[w.index("grid") + 1]) <= 152
+    assert int(w[w.index("smem") + 1]) >= 200 * 1024
