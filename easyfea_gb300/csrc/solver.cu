@@ -2039,7 +2039,7 @@ int fetch(Scal* h, PcgWork& w, cudaStream_t st) {
 // Whether this solve runs as one resident launch (resident.cu): an operator
 // that is not staged (its tiles would fit in half of the L2), host checks left
 // to the library, and nothing that needs the iteration's launches one by one
-// (kernel timing, a first solve that tunes the SpMV, the direct-launch entry).
+// (kernel timing, the direct-launch entry, a number of lanes for its product).
 //
 // Its CTAs, one per SM, must all run at once: the grid is bounded by the
 // device's SMs (an MPS share's, where the context has one), and a launch that
@@ -2047,15 +2047,12 @@ int fetch(Scal* h, PcgWork& w, cudaStream_t st) {
 // multi-kernel iteration.
 template <typename T>
 bool use_resident(const gfea_system* s, const gfea_pcg_opts* o, const PcgWork& w, bool direct_only, ResidentGeom* g) {
-  if (direct_only || !w.box || o->check_every > 0 || prof().on.load()) return false;
+  if (direct_only || !w.box || o->check_every > 0 || o->lanes > 0 || prof().on.load()) return false;
   static const bool off = [] {
     const char* v = getenv("GFEA_RESIDENT");  // "0": the multi-kernel iteration
     return v && v[0] == '0';
   }();
   if (off) return false;
-  int32_t tuned = 0;
-  if (o->lanes == 0 && tune_cache().mode.load() == 2 && !tune_get(spmv_key(s, sizeof(T) == 4 ? GFEA_F32 : GFEA_F64), &tuned))
-    return false;
   // Solves in flight share the SMs: a cooperative grid starts when all its
   // CTAs fit, so full-size grids would run one after the other, each bound by
   // latency (24 served requests: 55 ms with full-size grids, 39 ms with a
@@ -2144,6 +2141,23 @@ int refine_solve(const gfea_system* s, const double* b, double* x, const gfea_pc
       for (int i = 0; i < 3; ++i) cudaEventDestroy(ev[i]);
     }
   }
+  int32_t tuned = 0;
+  if (!direct_only && o->lanes == 0 && tune_cache().mode.load() == 2 && !tune_get(spmv_key(s, vt), &tuned)) {
+    // first solve of this problem class: time the PCG's own SpMV kernel on the
+    // initial residual (also where this solve is a resident one: reactions and
+    // products of the class read the schedule), then reset the scalar record
+    e = launch_resid(s, G, b, x, w, false, st);
+    if (e) return e;
+    e = fetch(&hs, w, st);
+    if (e) return e;
+    if (hs.rr_true > 0) {
+      cast_kernel<T><<<grid_elems(N), kThreads, 0, st>>>(w.r64, (T*)w.pa, N);
+      GFEA_LAUNCH_CHECK();
+      e = tune_apply_impl<T>(s, w, st, &G);
+      if (e) return e;
+    }
+    GFEA_CUDA_TRY(cudaMemsetAsync(w.sc, 0, sizeof(Scal), st));
+  }
   ResidentGeom geom;
   if (use_resident<T>(s, o, w, direct_only, &geom)) {
     // pa and pb are adjacent: the packets of p; rcp holds three accumulators
@@ -2198,17 +2212,6 @@ int refine_solve(const gfea_system* s, const double* b, double* x, const gfea_pc
   e = fetch(&hs, w, st);
   if (e) return e;
   if (flag) { res->status = GFEA_ERR_SINGULAR; return GFEA_ERR_SINGULAR; }
-  int32_t tuned = 0;
-  if (!direct_only && o->lanes == 0 && tune_cache().mode.load() == 2 && !tune_get(spmv_key(s, vt), &tuned) &&
-      hs.rr_true > 0) {
-    // first solve of this problem class: time the PCG's own SpMV kernel on the
-    // initial residual, then reset the scalar record it wrote
-    cast_kernel<T><<<grid_elems(N), kThreads, 0, st>>>(w.r64, (T*)w.pa, N);
-    GFEA_LAUNCH_CHECK();
-    e = tune_apply_impl<T>(s, w, st, &G);
-    if (e) return e;
-    GFEA_CUDA_TRY(cudaMemsetAsync(w.sc, 0, sizeof(Scal), st));
-  }
   const double bb = hs.bb;
   if (!(bb == bb) || !isfinite(hs.rr_true)) { res->status = GFEA_ERR_NAN; return GFEA_ERR_NAN; }
   if (bb == 0) {  // b_i - A_ic x_c = 0: the unknowns are zero

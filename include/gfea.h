@@ -351,7 +351,8 @@ typedef struct gfea_pcg_opts {
                                residual replacements (reliable updates); outside (0, 1):
                                0.1 with block-Jacobi alone, 0.01 with the coarse level */
   int32_t max_refine;       /* refinement steps cap (mixed precision) */
-  int32_t lanes;            /* SpMV lanes per node (0 = automatic) */
+  int32_t lanes;            /* SpMV lanes per node of the multi-kernel iteration (0 =
+                               automatic; a number asks for that iteration) */
   int32_t coarse;           /* two-level preconditioner: target number of aggregates
                                (0 = block-Jacobi only, -1 = automatic); needs sys.coord */
   int32_t coarse_reuse;     /* 1: the workspace holds the aggregation of an earlier call

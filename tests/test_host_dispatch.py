@@ -113,3 +113,18 @@ def test_long_rows_spread_over_more_ctas(run, nodes, degree, precision, least):
     w = line.split()
     assert least <= int(w[w.index("grid") + 1]) <= 152
     assert int(w[w.index("smem") + 1]) >= 200 * 1024
+
+
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+def test_lanes_reach_the_product_they_schedule(run, precision):
+    (s,) = run({**BOX, "precision": precision, "lanes": 16})
+    assert "resident_kernel" not in names(s) and any(n.startswith("apply") for n in names(s))
+
+
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+def test_first_solve_tunes_the_product_and_is_resident(run, precision):
+    first, second = run({**BOX, "precision": precision, "tune_mode": 2}, {**BOX, "precision": precision, "tune_mode": 2})
+    n = names(first)
+    assert any(k.startswith("apply") for k in n[:n.index("resident_kernel")])
+    assert n[-1] == "resident_kernel" == names(second)[-1]
+    assert not any(k.startswith("apply") for k in names(second))
