@@ -8,6 +8,20 @@
 
 namespace gfea {
 
+// Regularisation of a coarse matrix R^T K R, relative to its largest diagonal
+// entry: one at most zero_tol is replaced by the largest (empty or fully
+// constrained unknowns), the others are shifted (rotations of degenerate
+// aggregates).  FP32 values: their rounding reaches the 1e-6 level in nearly
+// degenerate modes.  FP64: 1e-8 keeps those modes well above the float-float
+// rounding of the inversion (~1e-12 of the largest entry, times the growth
+// over the pivot blocks); at 1e-10 the inverse of a 64-aggregate HEXA8 bar
+// comes out indefinite, also with its pivot blocks in FP64.  Iterations are
+// the same with either.
+struct CoarseReg {
+  double zero_tol, shift;
+};
+inline CoarseReg coarse_reg(bool f32) { return f32 ? CoarseReg{1e-6, 1e-6} : CoarseReg{1e-14, 1e-8}; }
+
 inline int coarse_nr(int D) { return D == 1 ? 1 : (D == 2 ? 3 : 6); }
 
 // Aggregation kept at the start of the coarse workspace, so that a later

@@ -590,11 +590,7 @@ __global__ void coarse_assemble_kernel(SysT<T> S, CoarseDev C) {
   coarse_assemble_body<D, T>(S, C, blockIdx.x, gridDim.x);
 }
 
-// Unit diagonal for empty or fully constrained coarse DOFs, a 1e-10 relative
-// shift elsewhere (rotation modes of degenerate aggregates), identity in inv.
-// (zero_tol, shift) of a batch's matrices: (1e-14, 1e-10) for those built in FP64,
-// (1e-6, 1e-6) for one built from FP32 values, whose rounding can reach the
-// 1e-6 level in nearly degenerate modes.
+// A batch's regularisation (see coarse_reg).
 __device__ __forceinline__ void coarse_regularize_body(const CoarseDev& C, double zero_tol, double shift) {
   __shared__ double smax[256];
   double m = 0;
@@ -1739,12 +1735,8 @@ int coarse_matrix(const gfea_system* s, CoarseDev& C, cudaStream_t st, cudaEvent
   GFEA_D_SWITCH(D, (coarse_assemble_kernel<DD, T><<<grid_elems(Nn * coarse_nr(D)), kThreads, 0, st>>>(S, C)));
   GFEA_LAUNCH_CHECK();
   if (mark) GFEA_CUDA_TRY(cudaEventRecord(mark, st));
-  // FP64 values: the shift keeps nearly degenerate modes (rotations of one-
-  // or two-node aggregates) well above the float-float rounding of the
-  // inversion (~1e-12 of the largest entry): at 1e-10 the 384-unknown coarse
-  // matrix of a 64-aggregate HEXA8 bar came out indefinite; iterations are the
-  // same with either.
-  return sizeof(T) == 4 ? coarse_inverse(C, 1e-6, 1e-6, st) : coarse_inverse(C, 1e-14, 1e-8, st);
+  const CoarseReg reg = coarse_reg(sizeof(T) == 4);
+  return coarse_inverse(C, reg.zero_tol, reg.shift, st);
 }
 
 template <typename T>
@@ -2708,10 +2700,8 @@ extern "C" int gfea_coarse_batch_build(const void* scratch, int n, const int32_t
     }
     GFEA_LAUNCH_CHECK();
   }
-  if (precision == GFEA_F32)
-    cb_regularize_kernel<<<n, 256, 0, st>>>(jobs, 1e-6, 1e-6);
-  else
-    cb_regularize_kernel<<<n, 256, 0, st>>>(jobs, 1e-14, 1e-10);
+  const CoarseReg reg = coarse_reg(precision == GFEA_F32);
+  cb_regularize_kernel<<<n, 256, 0, st>>>(jobs, reg.zero_tol, reg.shift);
   GFEA_LAUNCH_CHECK();
   cb_split_kernel<<<dim3(ge, n), kThreads, 0, st>>>(jobs);
   GFEA_LAUNCH_CHECK();
