@@ -6,6 +6,8 @@
 
 #include <cstdint>
 
+#include "rowops.cuh"
+
 namespace gfea {
 
 template <int D>
@@ -39,6 +41,22 @@ __device__ __forceinline__ void node_modes(float4 o, const uint8_t* kn, T (&R)[D
       R[1][m] = k1 ? T(0) : r1[m];
       R[2][m] = k2 ? T(0) : r2[m];
     }
+  }
+}
+
+// acc += R[:, m]^T x over the components x of a node at offset o (unmasked): the
+// mode's non-zero products.
+template <int D, typename T>
+__host__ __device__ __forceinline__ void add_mode(DotAcc<T>& acc, int m, const T* o, const T* x) {
+  if (D == 1 || m < D) {
+    acc.add(x[m]);
+  } else if constexpr (D == 2) {
+    acc.add_prod(o[0], x[1]);
+    acc.add_prod(-o[1], x[0]);
+  } else if constexpr (D == 3) {
+    const int a = m - 3, b = a == 2 ? 0 : a + 1, c = a == 0 ? 2 : a - 1;  // rotation about axis a
+    acc.add_prod(o[b], x[c]);
+    acc.add_prod(-o[c], x[b]);
   }
 }
 

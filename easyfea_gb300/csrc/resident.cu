@@ -42,7 +42,9 @@
 //
 // FP64 instructions retire at a sixteenth of a warp per cycle and SM, so the
 // scalar recurrences run in one thread, the sums of the partials in one warp
-// per value, and the restriction sums each aggregate's nodes directly.
+// per value, and the restriction sums each aggregate's nodes directly (in
+// float pairs in the FP32 solve: a CTA's share of an aggregate may be hundreds
+// of nodes).
 #include <math.h>
 #include <stdlib.h>
 
@@ -312,20 +314,6 @@ __device__ __forceinline__ void load_block(const T* b, T (&v)[D]) {
 #pragma unroll
     for (int d = 0; d < D; ++d) v[d] = b[d];
   }
-}
-
-// The non-zero products of rigid-body mode m: v = c1 x[k1] + c2 x[k2] over the
-// components x of a node at offset o (k1 = -1: one component, x[m]).
-template <int D, typename T>
-__device__ __forceinline__ T mode_product(int m, const T* o, const T* x) {
-  if (D == 1 || m < D) return x[m];
-  if constexpr (D == 2) {
-    return o[0] * x[1] - o[1] * x[0];
-  } else if constexpr (D == 3) {
-    const int a = m - 3, b = a == 2 ? 0 : a + 1, c = a == 0 ? 2 : a - 1;  // rotation about axis a
-    return o[b] * x[c] - o[c] * x[b];
-  }
-  return 0;
 }
 
 // Component k of R e at offset o (e: the modes' coefficients).
@@ -605,7 +593,7 @@ __global__ void __launch_bounds__(kRT, 1) resident_kernel(ResidentProblem<T> P, 
     const int tasks = s_nseg * nr, h = tid % H;
     for (int t0 = 0; t0 < tasks; t0 += kRT / H) {
       const int t = t0 + tid / H;
-      T v = 0;
+      DotAcc<T> v;
       int g = 0, m = 0;
       if (t < tasks) {
         const int l = t / nr;
@@ -614,15 +602,15 @@ __global__ void __launch_bounds__(kRT, 1) resident_kernel(ResidentProblem<T> P, 
         const int k1 = seg_ptr[l + 1];
         for (int k = seg_ptr[l] + h; k < k1; k += H) {
           const int i = order_s[k];
-          v += mode_product<D, T>(m, off_s + i * D, v_s + i * D);
+          add_mode<D, T>(v, m, off_s + i * D, v_s + i * D);
         }
       }
-      for (int o = H >> 1; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+      const double sum = warp_sum_acc(v, H);
       if (t < tasks && h == 0) {
         if (solo)
-          sv_s[g * nr + m] = (double)v;
+          sv_s[g * nr + m] = sum;
         else
-          atomicAdd(s_now + g * nr + m, (double)v);
+          atomicAdd(s_now + g * nr + m, sum);
       }
     }
   };
@@ -979,7 +967,7 @@ __global__ void __launch_bounds__(kRT, 1) resident_kernel(ResidentProblem<T> P, 
         } else {
           Pk::store(P.ec + 2 * i, (T)v, ec_number);
         }
-        w[0] += v * rc_s[i];
+        w[0] += (double)(T)v * rc_s[i];  // r.z of the z that takes ec rounded to T
       }
     }
     ok = exchange<2, false>(

@@ -26,14 +26,21 @@ struct SysT {
 template <typename T>
 struct DotAcc {
   double v = 0;
-  __device__ __forceinline__ void add_prod(T a, T b) { v += (double)a * (double)b; }
-  __device__ __forceinline__ double value() const { return v; }
+  __host__ __device__ __forceinline__ void add(T a) { v += (double)a; }
+  __host__ __device__ __forceinline__ void add_prod(T a, T b) { v += (double)a * (double)b; }
+  __host__ __device__ __forceinline__ double value() const { return v; }
 };
 
 template <>
 struct DotAcc<float> {
   float s = 0.f, c = 0.f;
-  __device__ __forceinline__ void add_prod(float a, float b) {
+  __host__ __device__ __forceinline__ void add(float a) {
+    const float t = s + a;
+    const float bp = t - s;
+    c += (s - (t - bp)) + (a - bp);
+    s = t;
+  }
+  __host__ __device__ __forceinline__ void add_prod(float a, float b) {
     const float p = a * b;
     const float e = fmaf(a, b, -p);
     const float t = s + p;
@@ -42,24 +49,25 @@ struct DotAcc<float> {
     s = t;
     c += err + e;
   }
-  __device__ __forceinline__ double value() const { return (double)s + (double)c; }
+  __host__ __device__ __forceinline__ double value() const { return (double)s + (double)c; }
 };
 
-// Warp sum of dot accumulators (every lane receives it).  FP32 pairs are
+// Sum of dot accumulators over a warp, or over aligned groups of 'lanes' lanes
+// (every lane receives it).  FP32 pairs are
 // combined with TwoSum at each butterfly step, so the sum keeps the pairs'
 // accuracy with one FP64 conversion per lane instead of FP64 shuffles and
 // adds (GB300's FP64 pipe made those a visible share of short kernels).
-__device__ __forceinline__ double warp_sum_acc(const DotAcc<double>& a) {
+__device__ __forceinline__ double warp_sum_acc(const DotAcc<double>& a, int lanes = 32) {
   double v = a.v;
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  for (int o = lanes >> 1; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
   return v;
 }
 
-__device__ __forceinline__ double warp_sum_acc(const DotAcc<float>& a) {
+__device__ __forceinline__ double warp_sum_acc(const DotAcc<float>& a, int lanes = 32) {
   float s = a.s, c = a.c;
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
+  for (int o = lanes >> 1; o > 0; o >>= 1) {
     const float s2 = __shfl_xor_sync(0xffffffffu, s, o), c2 = __shfl_xor_sync(0xffffffffu, c, o);
     const float t = s + s2;
     const float bp = t - s;

@@ -782,7 +782,10 @@ __global__ void __launch_bounds__(kThreads) rc_sum_kernel(CoarseDev C, const Sca
 // blocks of several rows: with one row a block, the 1,152 tickets and
 // partials of the 2.02M-unknown box's coarse level took a third of the kernel
 // (16.9 us one row a block, 13.7 us four).
+//
+// F32: the FP32 iteration, whose z takes ec rounded to FP32; rc.ec does too.
 constexpr int kGemvThreads = 128, kGemvRows = 4;
+template <bool F32>
 __global__ void __launch_bounds__(kGemvThreads* kGemvRows)
     coarse_gemv_kernel(CoarseDev C, double* partials, Scal* sc, int mode) {
   if (mode == 0 && sc->done) return;
@@ -807,7 +810,7 @@ __global__ void __launch_bounds__(kGemvThreads* kGemvRows)
       for (int w = 0; w < kWarps; ++w) t += sh[sub * kWarps + w];
       C.ec[i] = t;
       C.ecf[i] = (float)t;
-      dot[0] += t * C.rc[i];
+      dot[0] += (F32 ? (double)(float)t : t) * C.rc[i];
     }
     __syncthreads();
   }
@@ -1630,7 +1633,7 @@ int launch_precond(const gfea_system* s, PcgWork& w, T* x, T* p, int mode, cudaS
     rc_sum_kernel<<<(int)ceil_div(w.C.nc, kThreads), kThreads, 0, st>>>(w.C, w.sc, mode);
     GFEA_LAUNCH_CHECK();
   }
-  coarse_gemv_kernel<<<(int)std::min<int64_t>(ceil_div(w.C.nc, kGemvRows), 8 * kSMs), kGemvThreads * kGemvRows, 0, st>>>(
+  coarse_gemv_kernel<sizeof(T) == 4><<<(int)std::min<int64_t>(ceil_div(w.C.nc, kGemvRows), 8 * kSMs), kGemvThreads * kGemvRows, 0, st>>>(
       w.C, w.partials, w.sc, mode);
   GFEA_LAUNCH_CHECK();
   e = prof_mark(st, kTagGemv);
