@@ -2032,7 +2032,10 @@ int fetch(Scal* h, PcgWork& w, cudaStream_t st) {
 }
 
 // Whether this solve runs as one resident launch (resident.cu): an operator
-// that is not staged (its tiles would fit in half of the L2), host checks left
+// that is small enough not to be staged (its tiles would fit in half of the
+// L2) or whose tiles are too large for that (rows of 31 neighbours and more in
+// FP64 3D, 62 in FP32) but which has at most kResidentPairs stored blocks a
+// CTA, host checks left
 // to the library, and nothing that needs the iteration's launches one by one
 // (kernel timing, the direct-launch entry, a number of lanes for its product).
 //
@@ -2040,6 +2043,15 @@ int fetch(Scal* h, PcgWork& w, cudaStream_t st) {
 // device's SMs (an MPS share's, where the context has one), and a launch that
 // is refused all the same (a green context) leaves the solve to the
 // multi-kernel iteration.
+//
+// Beyond kResidentPairs the part of p that a CTA of corner nodes reads no longer
+// fits beside its rows' indices, and the solve falls behind the multi-kernel
+// iteration.  FP64 at 152 CTAs, resident and multi-kernel ms: 32,721 PRISM15
+// nodes (8,710 blocks a CTA) 21.8 and 27.3, 23,373 HEXA27 (9,030) 15.7 and 15.7,
+// 32,193 PRISM18 (9,030) 26.0 and 18.9, 26,481 HEXA20 (9,210) 21.4 and 23.4,
+// 29,081 HEXA20 (10,100) 32.9 and 24.5, 26,901 HEXA27 (10,400) 27.9 and 15.8.
+constexpr int64_t kResidentPairs = 9000;
+
 template <typename T>
 bool use_resident(const gfea_system* s, const gfea_pcg_opts* o, const PcgWork& w, bool direct_only, ResidentGeom* g) {
   if (direct_only || !w.box || o->check_every > 0 || o->lanes > 0 || prof().on.load()) return false;
@@ -2058,8 +2070,12 @@ bool use_resident(const gfea_system* s, const gfea_pcg_opts* o, const PcgWork& w
       cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
     return false;
   sms = std::min(sms, kSMs);  // the packets' room
-  return resident_geom<T>(s->dof_n, s->n_nodes, s->n_pairs, w.coarse ? w.C.nc : 0, w.coarse ? w.C.n_agg : 0,
-                          std::max(sms / active, 1), g);
+  if (packed_bytes<T>(s) > 0) return false;  // a staged operator without the room for its tiles
+  if (!resident_geom<T>(s->dof_n, s->n_nodes, s->n_pairs, w.coarse ? w.C.nc : 0, w.coarse ? w.C.n_agg : 0,
+                        std::max(sms / active, 1), g))
+    return false;
+  StageGeom tiles;
+  return stage_geom<T>(s, sys_t<T>(s).vals, &tiles) || s->n_pairs <= kResidentPairs * g->grid;
 }
 
 // PCG in T precision with reliable updates (FP64 residual replacement):

@@ -43,7 +43,11 @@ def main(fake_path, steps):
         opts = _lib.PcgOpts(_lib.ABI_VERSION, prec, 100, s.get("check_every", 0), 1e-10, 0.0, 10, s.get("lanes", 0),
                             s.get("coarse", -1), 0)
         ws = ctypes.c_size_t()
+        if s.get("work_without_tiles"):  # the size that a smaller threshold's operator would need
+            os.environ["GFEA_STAGE_MIN_BYTES"] = str(1 << 60)
         assert L.gfea_pcg_workspace_size(ctypes.byref(sysd), ctypes.byref(opts), ctypes.byref(ws)) == 0
+        os.environ.pop("GFEA_STAGE_MIN_BYTES", None)
+        os.environ.update(s.get("env", {}))
         work = np.zeros(ws.value + 256, np.uint8)
         base = (work.ctypes.data + 255) & ~255
         res = _lib.PcgResult()

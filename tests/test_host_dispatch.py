@@ -128,3 +128,22 @@ def test_first_solve_tunes_the_product_and_is_resident(run, precision):
     assert any(k.startswith("apply") for k in n[:n.index("resident_kernel")])
     assert n[-1] == "resident_kernel" == names(second)[-1]
     assert not any(k.startswith("apply") for k in names(second))
+
+
+@pytest.mark.parametrize("nodes,degree,precision,resident", [
+    (13005, 57, "fp64", True), (26901, 59, "fp64", False), (69000, 64, "fp64", False), (38360, 53, "fp64", False),
+    (20280, 52, "fp64", True), (22000, 58, "mixed", True), (60000, 60, "mixed", False), (2000, 8, "fp64", True)])
+def test_operators_that_cannot_be_staged_are_resident_up_to_a_size(run, nodes, degree, precision, resident):
+    """Tiles of long rows are too large to be staged at any size: that they are
+    not staged does not mean that they stay in L2."""
+    (s,) = run({**BOX, "nodes": nodes, "degree": degree, "precision": precision, "coarse": 0})
+    assert ("resident_kernel" in names(s)) == resident
+    assert resident or any(n.startswith("apply") for n in names(s))
+
+
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+def test_staged_operator_in_a_workspace_without_tiles_is_not_resident(run, precision):
+    big = {**BOX, "nodes": 90000, "precision": precision, "coarse": 0}
+    s, short = run(big, {**big, "work_without_tiles": 1})
+    assert "apply_staged_kernel" in names(s)
+    assert "resident_kernel" not in names(short) and "apply_kernel" in names(short)
