@@ -28,7 +28,6 @@ struct ResidentProblem {
   int coarse;         // two-level preconditioner
   double* box;        // packets of the partial sums (zero at launch)
   ResidentOut* out;   // zero at launch
-  uint64_t wait_ns;   // limit of every wait
   double rtol, delta2;
   int max_iters, max_upd;
 };

@@ -2185,7 +2185,6 @@ int refine_solve(const gfea_system* s, const double* b, double* x, const gfea_pc
     P.box = reinterpret_cast<double*>(w.box);
     static_assert(sizeof(ResidentOut) <= sizeof(Scal), "the scalar record's place");
     P.out = reinterpret_cast<ResidentOut*>(w.sc);
-    P.wait_ns = kWaitLimitNs;
     P.rtol = o->rtol;
     P.delta2 = delta2;
     P.max_iters = o->max_iters;
