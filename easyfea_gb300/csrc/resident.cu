@@ -1087,18 +1087,22 @@ int launch(const ResidentProblem<T>& P, const ResidentGeom& g, cudaStream_t st) 
 
 }  // namespace
 
-// Rows per CTA: enough to keep its threads busy, few enough to use many SMs;
-// of long rows no more than 10,240 values (a HEXA8's 128 rows), by which a CTA's
-// time goes.  Shared memory: all of it.  Numberings that take the corner nodes
-// first (every quadratic 3D mesh) give the first CTAs rows of twice the average
-// length, which room for the average left to L2.  In FP64, average room and 128
-// rows -> this, beside the multi-kernel iteration's: 425 HEXA27 nodes 4.75 -> 2.44
-// ms (3.22), 2,025 8.42 -> 3.99 (6.31), 600 HEXA20 6.21 -> 3.19 (4.79), 2,025
-// PRISM18 7.68 -> 3.87 (5.60), 2,025 TETRA10 6.71 -> 3.56 (6.11).
+// Rows per CTA: enough to keep its threads busy, few enough to use many SMs; in
+// 3D no more than 10,240 values (of HEXA8 139 rows, of HEXA27 65), by which a
+// CTA's time goes there.  (In 2D more CTAs cost more in exchanges than they
+// save: 12,261 TRI15 nodes, FP32, 96 CTAs 4.9 ms, 111 5.2, 152 5.4.)  Shared
+// memory: room for rows of two (2D) and three times the average length.
+// Numberings that take the corner nodes first (every quadratic mesh) give the
+// first CTAs the long rows, which room for the average left to L2; all of it for
+// every solve is 0.5 % slower.  In FP64, average room and 128 rows -> this, beside
+// the multi-kernel iteration's: 425 HEXA27 nodes 4.75 -> 2.42 ms (3.22), 2,025
+// 8.42 -> 3.97 (6.31), 600 HEXA20 6.21 -> 3.20 (4.79), 2,025 PRISM18 7.68 -> 3.82
+// (5.60), 2,025 TETRA10 6.71 -> 3.61 (6.11).
 template <typename T>
 bool resident_geom(int D, int64_t Nn, int64_t n_pairs, int nc, int n_agg, int sms, ResidentGeom* g) {
   const double nb = (double)n_pairs / (double)Nn;
-  const int64_t rows = std::min<int64_t>(sizeof(T) == 8 ? 128 : 256, std::max<int64_t>(32, (int64_t)(10240 / (nb * D))));
+  int64_t rows = sizeof(T) == 8 ? 128 : 256;
+  if (D == 3) rows = std::min<int64_t>(rows, std::max<int64_t>(32, (int64_t)(10240 / (nb * D))));
   if (const char* e = getenv("GFEA_RESIDENT_CTAS"))  // fewer, larger CTAs
     if (atoi(e) > 0) sms = std::min(sms, atoi(e));
   int64_t grid = ceil_div(Nn * D, rows);
@@ -1110,7 +1114,9 @@ bool resident_geom(int D, int64_t Nn, int64_t n_pairs, int nc, int n_agg, int sm
   if (n_agg > kAggWords * 32) return false;
   const size_t fixed = Layout<T>(D, g->npc, nc, n_agg, g->grid == 1).total;
   if (fixed > kRSmemMax / 2) return false;
-  g->smem = kRSmemMax;
+  const double want = (double)fixed + (D == 3 ? 3.0 : 2.0) * npc * nb * (sizeof(T) * D * D + 2) +
+                      (4 + sizeof(T) * D) * std::min<double>((double)Nn, npc * nb) + 8.0 * nc * (nc / g->grid + 1) + 4096;
+  g->smem = (size_t)std::min<double>(want, (double)kRSmemMax);
   // lanes per node by the row length, as in the multi-kernel SpMV
   const double W = D * nb;
   g->lanes = D == 1 ? (W <= 10 ? 4 : 8) : (D == 2 ? (W <= 24 ? 8 : 16) : (W <= 56 ? 16 : 32));
