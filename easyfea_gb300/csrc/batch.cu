@@ -16,7 +16,8 @@
 // of 2000 to 50000 unknowns, mixed precision, assembly included: 26.8 ms with
 // one neighbour pass and one node at a time and 256 threads throughout, 23.9
 // with the batched loads, 16.8 with the wide clusters; 64 of 3000 unknowns
-// 9.2 -> 7.3 ms, 256 of 2000 to 200000 276 -> 228 ms.
+// 9.2 -> 7.3 ms, 256 of 2000 to 200000 (10.9 million in all) 276 -> 228 ms, the
+// 256 random-material cantilevers of the benchmark (13.3 million) 351 -> 285.
 //
 // Cross-CTA reads of vectors written inside the launch use L2-only loads
 // (ld.global.cg), so no stale L1 line is ever consulted; the cluster barrier
@@ -46,9 +47,9 @@ constexpr int kCL = 8;    // CTAs per cluster (portable cluster size)
 // 5.4 -> 4.8 ms), but 8 whole SMs a cluster leave SMs unused and small systems
 // wait on barriers.  2000 to 50000 unknowns, 32 systems: 22.0 ms narrow, 16.2
 // wide; to 60000, 40 systems: 29.7 and 20.3, 100 systems: 40.0 and 43.2; 64 of
-// 3000: 7.3 and 13.3; 256 of 2000 to 200000: 228 and 280.  So: wide where the
-// largest system is over twice its share of the batch (the time of the batch
-// on all narrow clusters).
+// 3000: 7.3 and 13.3; 256 of 2000 to 200000 (10.9 million): 228 and 280.  So:
+// wide where the largest system is over twice its share of the batch (the time
+// of the batch on all narrow clusters).
 //
 // Both widths divide a system among the same kCL * 512 virtual threads, of
 // which a thread of the narrow one is two (VT, kWide / VT apart), and sum

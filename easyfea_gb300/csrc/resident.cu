@@ -27,18 +27,21 @@
 // readers enter once they have read it (partial sums, read and published at
 // the same exchanges, alternate between two sets).  Only what is not in
 // packets (the sums s, x after an update) is ordered by fences around the
-// exchange of the partial sums (1).  Every CTA adds the partials in the same order, so all take the same
-// decisions (convergence, updates, stopping) without the host.  The launch is
-// cooperative (the CTAs are co-resident); every poll is bounded: after 2 s (a
-// context suspended that long) the launch ends and reports it, and the host
-// goes on with the multi-kernel iteration, which waits for nothing.
+// exchange of the partial sums (1).  Every CTA adds the partials in the same
+// order, so all take the same decisions (convergence, updates, stopping)
+// without the host.  The launch is cooperative (the CTAs are co-resident);
+// every poll is bounded: after 2 s (a context suspended that long) the launch
+// ends and reports it, and the host goes on with the multi-kernel iteration,
+// which waits for nothing.
 //
 // Bound: latency (three exchanges of ~2 us, the halo, the serial chains
 // between them); in FP64 3D also the FP64 pipe (27 x 9 products per node: 5 us
 // of the 25 us iteration at 13,104 nodes).  Whole solves, multi-kernel ->
-// resident: 208 unknowns FP64 1.82 -> 1.02 ms, QUAD4 240x26 FP64 4.61 -> 2.50,
-// HEXA8 77x13x11 FP64 8.07 -> 4.06, QUAD9 461x50 mixed 15.6 -> 11.2, load
-// step of the 80,000-triangle plate 12.7 -> 7.9.
+// resident: 208 unknowns FP64 1.82 -> 0.99 ms, QUAD4 240x26 FP64 4.61 -> 2.16,
+// HEXA8 77x13x11 FP64 8.07 -> 3.44, QUAD9 461x50 mixed 15.6 -> 9.5, load step
+// of the 80,000-triangle plate 12.7 -> 6.7 (counters: barrier stalls of the
+// warps that wait for the polling one, 20 to 27 per issue; QUAD9 5.8 and 40 MB
+// an iteration from L2).
 //
 // FP64 instructions retire at a sixteenth of a warp per cycle and SM, so the
 // scalar recurrences run in one thread, the sums of the partials in one warp
@@ -69,7 +72,6 @@ template <typename T>
 struct Packet;
 template <>
 struct Packet<float> {
-  static constexpr int kWords = 2;  // of sizeof(float)
   static __device__ __forceinline__ void store(float* p, float v, uint32_t tag) {
     const uint64_t w = (uint64_t)tag << 32 | __float_as_uint(v);
     asm volatile("st.relaxed.gpu.global.b64 [%0], %1;" ::"l"(p), "l"(w) : "memory");
@@ -83,7 +85,6 @@ struct Packet<float> {
 };
 template <>
 struct Packet<double> {
-  static constexpr int kWords = 2;
   static __device__ __forceinline__ void store(double* p, double v, uint32_t tag) {
     asm volatile("{\n\t.reg .b128 w;\n\tmov.b128 w, {%1, %2};\n\tst.relaxed.gpu.global.b128 [%0], w;\n\t}" ::"l"(p),
                  "l"(__double_as_longlong(v)), "l"((uint64_t)tag)

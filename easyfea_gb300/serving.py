@@ -10,8 +10,11 @@ kinds and sizes arrive over time and share the device:
   footprint fits the remaining budget (a request that does not fit waits;
   smaller ones behind it may pass, up to ``max_bypass`` times).  Admitted
   requests run concurrently: their assembly and PCG launches interleave on
-  the device, and each solve keeps its own convergence test, so a result does
-  not depend on what else is running.
+  the device, and each solve keeps its own convergence test: its residual
+  meets the same bound whatever else is running.  (The grid of a resident
+  solve is its share of the SMs when it starts, and the coarse matrix is summed
+  with atomics, so the order of its sums, and with it the last digits, may
+  differ.)
 * Meshes (host arrays, device node graph, slot ranks) are built once per
   ``MeshSpec`` and stay resident; phase-field sessions keep their
   displacement, damage and history fields on the device between load steps.

@@ -342,9 +342,12 @@ typedef struct gfea_pcg_opts {
   int32_t version;          /* GFEA_ABI_VERSION */
   int32_t precision;        /* GFEA_F64: FP64 PCG; GFEA_F32: FP32 inner PCG + FP64 refinement */
   int32_t max_iters;        /* total PCG iteration cap */
-  int32_t check_every;      /* host convergence check period (iterations); <= 0: adaptive
-                               (first check after about as many iterations as the
-                               previous reliable-update cycle took, then doubling) */
+  int32_t check_every;      /* host convergence check period (iterations) of the
+                               multi-kernel iteration; <= 0: chosen by the library.  A
+                               solve whose operator stays on the chip then runs in one
+                               resident launch without host checks; others are checked
+                               every 8 iterations (staged operators) or first after about
+                               as many as the last reliable-update cycle took */
   double rtol;              /* target ||P(b - A x)|| / ||P(b - A x_c)||; the solve
                                stops at max(rtol, rounding floor), see gfea_pcg_result */
   double inner_rtol;        /* FP32: reduction of the iterated residual between FP64
@@ -399,7 +402,9 @@ typedef struct gfea_batch_instance {
   int32_t version;          /* GFEA_ABI_VERSION */
   int32_t dof_n;
   int64_t n_nodes;
-  int64_t n_pairs;
+  int64_t n_pairs;          /* stored node pairs; with dof_n the order in which the systems
+                               are taken and whether a cluster runs one with 256 or 512
+                               threads per block (the same result, to the bit) */
   const int32_t* node_ptr;
   const int32_t* nbr;
   const double* vals64;     /* FP64 CSR values (residuals) */
